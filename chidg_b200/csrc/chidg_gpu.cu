@@ -987,6 +987,9 @@ extern "C" int chidg_gpu_matvec(chidg_gpu_matrix* A, const chidg_gpu_vector* x, 
 // ---------------------------------------------------------------------------
 namespace {
 
+// the FP32 factorisation's tensor-core kernels take blocks of up to this size
+constexpr int FACTOR32_SMALL = 136;
+
 // transposed LOCAL block: first LOCAL block of row (p,t) whose column is e
 // (type_domain_matrix.f90:592-627)
 int find_trans(const chidg_gpu_matrix* A, int p, int t, int e) {
@@ -996,16 +999,6 @@ int find_trans(const chidg_gpu_matrix* A, int p, int t, int e) {
 }
 
 }  // namespace
-
-// CHIDG_FACTOR_TILES=1: factor products of blocks above 144 rows on the FP64
-// tensor cores in 136 x 136 tiles instead of the SIMT tiled kernel
-static bool factor_tiles_env() {
-    static const bool v = [] {
-        const char* e = std::getenv("CHIDG_FACTOR_TILES");
-        return e && e[0] == '1';
-    }();
-    return v;
-}
 
 // ILU0 / Jacobi on a single rank: one programme row per matrix row.
 static int build_ilu0(const chidg_gpu_matrix* A, bool jacobi, IluProgram& P, std::string& err) {
@@ -1379,14 +1372,14 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
     }
     // factorisation schedule per forward level.  Rows of a level are ordered
     // by block-size class so that each inverse launch uses the register tile
-    // that fits; GEMM tasks that fit one tensor-core CTA (<= 136 x 136) come
-    // first in each level.
+    // that fits; products of blocks that the FP32 tensor-core kernels take
+    // come first in each level.
     std::vector<GemmTask> ltasks, stasks;
     std::vector<GemmPair> lpairs, spairs;
     P.ltask_ptr.assign(P.fwd_ptr.size(), 0);
     P.stask_ptr.assign(P.fwd_ptr.size(), 0);
-    P.ltask_dmma.assign(P.fwd_ptr.size(), 0);
-    P.stask_dmma.assign(P.fwd_ptr.size(), 0);
+    P.ltask_small.assign(P.fwd_ptr.size(), 0);
+    P.stask_small.assign(P.fwd_ptr.size(), 0);
     P.inv_seg.clear();
     P.inv_seg_ptr.assign(P.fwd_ptr.size(), 0);
     const int nlev = (int)P.fwd_ptr.size() - 1;
@@ -1401,65 +1394,41 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
             i = j;
         }
         P.inv_seg_ptr[l + 1] = (int)P.inv_seg.size();
-        // pass 0: products on the FP64 tensor cores, one CTA per output block of
-        // up to 136 x 136 and, with CHIDG_FACTOR_TILES=1, one CTA per tile
-        // (r0, c0) of outputs of programmes whose blocks exceed 144 rows
-        // (the FP32 factorisation, which takes whole blocks up to 144, never
-        // sees a tile); pass 1: the larger outputs on the SIMT tiled kernel
-        // otherwise
-        const bool tiles = factor_tiles_env() && P.max_b > SF_MAX;
+        // pass 0: products of blocks of at most FACTOR32_SMALL rows (the FP32
+        // factorisation takes them on the tensor cores), pass 1: larger ones
         for (int pass = 0; pass < 2; ++pass) {
             for (int i = P.fwd_ptr[l]; i < P.fwd_ptr[l + 1]; ++i) {
                 const int pr = P.fwd_rows[i];
                 const int b = P.prow_b[pr];
-                // the tasks of one output (b rows, n columns): whole, or cut
-                // into balanced tiles of at most 136 x 136 (a multiple of 8
-                // rows and columns each, but the last)
-                auto span = [](int len) {
-                    const int parts = (len + DM_MAX - 1) / DM_MAX;
-                    return std::min(DM_MAX, ((len + parts - 1) / parts + 7) / 8 * 8);
-                };
-                auto add = [&](std::vector<GemmTask>& tasks, const GemmTask& t, int n, bool whole) {
-                    const int tm = whole ? b : span(b), tn = whole ? n : span(n);
-                    for (int r0 = 0; r0 < b; r0 += tm)
-                        for (int c0 = 0; c0 < n; c0 += tn) {
-                            GemmTask u = t;
-                            u.r0 = r0;
-                            u.c0 = c0;
-                            u.m = std::min(tm, b - r0);
-                            u.n = std::min(tn, n - c0);
-                            tasks.push_back(u);
-                        }
-                };
                 for (auto& en : P.lo[pr]) {
                     // L = A_lower * inv(D_parent)      (precon_ILU0.f90:231)
-                    const bool small = b <= DM_MAX && en.nc <= DM_MAX;
-                    if ((small || tiles) != (pass == 0)) continue;
+                    const bool small = b <= FACTOR32_SMALL && en.nc <= FACTOR32_SMALL;
+                    if (small != (pass == 0)) continue;
                     GemmTask t{};
-                    t.c_off = en.l_off; t.cinit_off = -1; t.ldm = b;
+                    t.c_off = en.l_off; t.cinit_off = -1; t.m = b; t.n = en.nc;
                     t.q_begin = (int32_t)lpairs.size();
                     lpairs.push_back(GemmPair{en.a_off, P.dinv_off[en.parent], en.nc, 0});
                     t.q_end = (int32_t)lpairs.size();
                     t.elem = P.prow_elem[pr];
-                    add(ltasks, t, en.nc, small || pass == 1);
+                    ltasks.push_back(t);
                 }
                 // D = A_diag - sum L * A(parent, itranspose)   (:238-239);
                 // assembled rows get their D from k_assemble_rows instead
                 if (P.assembled) continue;
-                bool small = b <= DM_MAX;
-                for (auto& en : P.lo[pr]) small = small && en.nc <= DM_MAX;
-                if ((small || tiles) != (pass == 0)) continue;
+                bool small = b <= FACTOR32_SMALL;
+                for (auto& en : P.lo[pr]) small = small && en.nc <= FACTOR32_SMALL;
+                if (small != (pass == 0)) continue;
                 GemmTask t{};
-                t.c_off = P.dinv_off[pr]; t.cinit_off = P.diagA_off[pr]; t.ldm = b;
+                t.c_off = P.dinv_off[pr]; t.cinit_off = P.diagA_off[pr]; t.m = b; t.n = b;
                 t.q_begin = (int32_t)spairs.size();
                 for (auto& en : P.lo[pr]) spairs.push_back(GemmPair{en.l_off, en.t_off, en.nc, 0});
                 t.q_end = (int32_t)spairs.size();
                 t.elem = P.prow_elem[pr];
-                add(stasks, t, b, small || pass == 1);
+                stasks.push_back(t);
             }
             if (pass == 0) {
-                P.ltask_dmma[l + 1] = (int)ltasks.size() - P.ltask_ptr[l];
-                P.stask_dmma[l + 1] = (int)stasks.size() - P.stask_ptr[l];
+                P.ltask_small[l + 1] = (int)ltasks.size() - P.ltask_ptr[l];
+                P.stask_small[l + 1] = (int)stasks.size() - P.stask_ptr[l];
             }
         }
         P.ltask_ptr[l + 1] = (int)ltasks.size();
@@ -1900,11 +1869,11 @@ static int factor_fp32(chidg_gpu_precon* M, chidg_gpu_matrix* A, int precision) 
     double* LD = (double*)M->LD.ptr;
     const int ph = prof_begin(ctx, kProfFactor);
     // products of blocks above 136 rows (the tasks after the first
-    // ltask_dmma / stask_dmma of a level): the SIMT tiled kernel in FP32
+    // ltask_small / stask_small of a level): the SIMT tiled kernel in FP32
     const int tiles_1d = (P.max_b + GT_M - 1) / GT_M;
     for (int l = 0; l < nlev; ++l) {
         const int pg = prof_begin(ctx, kProfFactorGemm);
-        const int nl_all = P.ltask_ptr[l + 1] - P.ltask_ptr[l], nl = P.ltask_dmma[l + 1];
+        const int nl_all = P.ltask_ptr[l + 1] - P.ltask_ptr[l], nl = P.ltask_small[l + 1];
         const int ns_all = P.stask_ptr[l + 1] - P.stask_ptr[l];
         const GemmTask* lt = (const GemmTask*)P.d_ltasks.ptr + P.ltask_ptr[l];
         const GemmTask* stt = (const GemmTask*)P.d_stasks.ptr + P.stask_ptr[l];
@@ -1925,7 +1894,7 @@ static int factor_fp32(chidg_gpu_precon* M, chidg_gpu_matrix* A, int precision) 
                     lt, 2 * nl, (const GemmPair*)P.d_lpairs.ptr, A32, L32, nullptr, L32, 1.0, wstat, kSpinLimit);
             if ((st = check_launch(ctx, "factor L products (FP32 / TF32)"))) return st;
         }
-        const int ns = P.stask_dmma[l + 1];
+        const int ns = P.stask_small[l + 1];
         if (ns_all > ns) {
             k_task_gemm<float, float, double, float><<<(ns_all - ns) * tiles_1d * tiles_1d, 256, 0, ctx->stream>>>(
                 stt + ns, (const GemmPair*)P.d_spairs.ptr, tiles_1d, tiles_1d, L32, A32, (const double*)A->val.ptr, LD, -1.0);
@@ -1994,8 +1963,7 @@ extern "C" int chidg_gpu_precon_update(chidg_gpu_precon* M, chidg_gpu_matrix* A,
     // error would otherwise leave them out of step)
     if (M->sync.ptr)
         cudaMemsetAsync((unsigned*)M->sync.ptr + 2 + P.nprow, 0, sizeof(unsigned) * 3 * (size_t)P.nprow, ctx->stream);
-    if ((precision == CHIDG_GPU_MIXED_FP32 || precision == CHIDG_GPU_MIXED_BF16) && !P.assembled &&
-        (P.max_b <= SF_MAX || !factor_tiles_env())) {
+    if ((precision == CHIDG_GPU_MIXED_FP32 || precision == CHIDG_GPU_MIXED_BF16) && !P.assembled) {
         // the inner solves only read FP32 / BF16 factors: compute them in FP32
         if ((st = factor_fp32(M, A, precision))) return st;
         cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
@@ -2016,9 +1984,9 @@ extern "C" int chidg_gpu_precon_update(chidg_gpu_precon* M, chidg_gpu_matrix* A,
         return CHIDG_GPU_OK;
     }
     const int nlev = (int)P.fwd_ptr.size() - 1;
-    const int tiles_1d = (P.max_b + GT_M - 1) / GT_M;
-    // one CTA per output block on the FP64 tensor cores for blocks up to 136 x 136
-    if ((st = raise_smem_limit((const void*)k_task_gemm_dmma<double, double, double>, DM_SMEM))) return fail(ctx, st, "factor GEMM shared memory");
+    // CTA tiles per side of the largest output (k_task_gemm_f64)
+    const int parts = fg_parts(P.max_b);
+    if ((st = raise_smem_limit((const void*)k_task_gemm_f64, FG_SMEM))) return fail(ctx, st, "factor GEMM shared memory");
     const int ph = prof_begin(ctx, kProfFactor);
     if (P.assembled) {
         k_assemble_rows<<<P.nprow, 256, 0, ctx->stream>>>((double*)M->LD.ptr, (const int64_t*)P.d_dinv_off.ptr,
@@ -2030,31 +1998,18 @@ extern "C" int chidg_gpu_precon_update(chidg_gpu_precon* M, chidg_gpu_matrix* A,
     }
     for (int l = 0; l < nlev; ++l) {
         const int pg = prof_begin(ctx, kProfFactorGemm);
-        const int nl = P.ltask_ptr[l + 1] - P.ltask_ptr[l], nld = P.ltask_dmma[l + 1];
-        if (nld > 0) {
-            k_task_gemm_dmma<double, double, double><<<nld, DM_THREADS, DM_SMEM, ctx->stream>>>(
-                (const GemmTask*)P.d_ltasks.ptr + P.ltask_ptr[l], (const GemmPair*)P.d_lpairs.ptr,
+        const int nl = P.ltask_ptr[l + 1] - P.ltask_ptr[l], ns = P.stask_ptr[l + 1] - P.stask_ptr[l];
+        if (nl > 0) {
+            k_task_gemm_f64<<<nl * parts * parts, FG_THREADS, FG_SMEM, ctx->stream>>>(
+                (const GemmTask*)P.d_ltasks.ptr + P.ltask_ptr[l], (const GemmPair*)P.d_lpairs.ptr, parts, parts,
                 (const double*)A->val.ptr, (const double*)M->LD.ptr, nullptr, (double*)M->LD.ptr, 1.0);
-            if ((st = check_launch(ctx, "k_task_gemm_dmma L"))) return st;
+            if ((st = check_launch(ctx, "k_task_gemm_f64 L"))) return st;
         }
-        if (nl > nld) {
-            k_task_gemm<double, double, double><<<(nl - nld) * tiles_1d * tiles_1d, 256, 0, ctx->stream>>>(
-                (const GemmTask*)P.d_ltasks.ptr + P.ltask_ptr[l] + nld, (const GemmPair*)P.d_lpairs.ptr, tiles_1d, tiles_1d,
-                (const double*)A->val.ptr, (const double*)M->LD.ptr, nullptr, (double*)M->LD.ptr, 1.0);
-            if ((st = check_launch(ctx, "k_task_gemm L"))) return st;
-        }
-        const int ns = P.stask_ptr[l + 1] - P.stask_ptr[l], nsd = P.stask_dmma[l + 1];
-        if (nsd > 0) {
-            k_task_gemm_dmma<double, double, double><<<nsd, DM_THREADS, DM_SMEM, ctx->stream>>>(
-                (const GemmTask*)P.d_stasks.ptr + P.stask_ptr[l], (const GemmPair*)P.d_spairs.ptr,
+        if (ns > 0) {
+            k_task_gemm_f64<<<ns * parts * parts, FG_THREADS, FG_SMEM, ctx->stream>>>(
+                (const GemmTask*)P.d_stasks.ptr + P.stask_ptr[l], (const GemmPair*)P.d_spairs.ptr, parts, parts,
                 (const double*)M->LD.ptr, (const double*)A->val.ptr, (const double*)A->val.ptr, (double*)M->LD.ptr, -1.0);
-            if ((st = check_launch(ctx, "k_task_gemm_dmma S"))) return st;
-        }
-        if (ns > nsd) {
-            k_task_gemm<double, double, double><<<(ns - nsd) * tiles_1d * tiles_1d, 256, 0, ctx->stream>>>(
-                (const GemmTask*)P.d_stasks.ptr + P.stask_ptr[l] + nsd, (const GemmPair*)P.d_spairs.ptr, tiles_1d, tiles_1d,
-                (const double*)M->LD.ptr, (const double*)A->val.ptr, (const double*)A->val.ptr, (double*)M->LD.ptr, -1.0);
-            if ((st = check_launch(ctx, "k_task_gemm S"))) return st;
+            if ((st = check_launch(ctx, "k_task_gemm_f64 S"))) return st;
         }
         prof_end(ctx, pg);
         const int pi = prof_begin(ctx, kProfFactorInv);

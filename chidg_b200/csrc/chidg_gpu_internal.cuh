@@ -2,6 +2,7 @@
 #pragma once
 #include "../../include/chidg_gpu.h"
 #include "kernels.cuh"
+#include "factor_gemm.cuh"
 #include "stream_sweep.cuh"
 #include "inverse_tc.cuh"
 #include "stream_matvec.cuh"
@@ -60,7 +61,8 @@ struct IluProgram {
     std::vector<std::vector<IluEntry>> lo, up;
     std::vector<int32_t> fwd_rows, bwd_rows;
     std::vector<int> fwd_ptr, bwd_ptr;
-    std::vector<int> ltask_ptr, stask_ptr, ltask_dmma, stask_dmma;
+    std::vector<int> ltask_ptr, stask_ptr;      // factor products per level
+    std::vector<int> ltask_small, stask_small;  // of them, those the FP32 kernels for small blocks take (first in the level)
     std::vector<std::array<int, 3>> inv_seg;   // per level: (row_begin, count, register-tile class)
     // task-split sweeps: tasks in hand-out order, partial offsets per entry
     int ntask_f = 0, ntask_b = 0;

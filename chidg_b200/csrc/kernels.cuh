@@ -427,10 +427,6 @@ struct GemmTask {            // C(m x n) = [Cinit] + sgn * sum_q A_q(m x k_q) B_
     int32_t m, n;
     int32_t q_begin, q_end;  // pairs
     int32_t elem;            // element id for status reporting
-    // k_task_gemm_dmma: the task may be the tile of rows r0.. and columns c0..
-    // of an output block of ldm rows (the A operands have ldm rows too);
-    // ldm = m, r0 = c0 = 0 for a whole block, which every other kernel takes
-    int32_t ldm, r0, c0;
 };
 struct GemmPair {
     int64_t a_off, b_off;
@@ -510,21 +506,6 @@ __global__ void __launch_bounds__(256) k_task_gemm(const GemmTask* __restrict__ 
     }
 }
 
-// FP64 tensor-core version of k_task_gemm for blocks up to 136 x 136: one CTA
-// computes a whole output block on the FP64 tensor cores (DMMA).  8 warps on
-// a 2 x 4 grid.  The 17 row tiles of 8 are taken in pairs (rows 16p ..
-// 16p+15, p < 8) by mma.sync m16n8k8, warp row wm owning pairs wm + 2i
-// (i < 4), and the last tile (rows 128..135) by m8n8k4 in warp row 0; warp
-// column wn owns the column tiles wn + 4j (j < 5).  Per slice of K = 8 a
-// warp loads its five B fragments once and each pair's A fragment once: 20
-// m16n8k8 (and 10 m8n8k4 in warp row 0) per slice, a third of the
-// instructions of the same work in m8n8k4.  K is staged 32 at a time through
-// shared memory in the same k-major layout for both operands, leading
-// dimension 140 (= 12 mod 16 doubles: the fragment loads of a half-warp hit
-// 16 distinct bank pairs); past the operands' K the stage holds zeros.
-constexpr int DM_MAX = 136, DM_LD = 140, DM_KC = 32, DM_WM = 2, DM_WN = 4, DM_TI = 9, DM_TJ = 5;
-constexpr int DM_THREADS = 32 * DM_WM * DM_WN;
-constexpr size_t DM_SMEM = 4 * sizeof(double) * DM_KC * DM_LD;   // two stages of (A, B) panels
 // 8-byte asynchronous global->shared copy; src_ok == false writes zeros
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool src_ok) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -537,127 +518,14 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // A(g+8, t+4); B(t, g), B(t+4, g); D(g, 2t), D(g, 2t+1), D(g+8, 2t), D(g+8, 2t+1)
 __device__ __forceinline__ void dmma_16x8x8(double& d0, double& d1, double& d2, double& d3, double a0, double a1,
                                             double a2, double a3, double b0, double b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+d"(d0), "+d"(d1), "+d"(d2), "+d"(d3)
                  : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
 }
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                  : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
-template <typename TA, typename TB, typename TC>
-__global__ void __launch_bounds__(DM_THREADS, 1) k_task_gemm_dmma(const GemmTask* __restrict__ tasks, const GemmPair* __restrict__ pairs,
-                                                               const TA* Abase, const TB* Bbase,
-                                                               const double* Cinit, TC* Cbase, double sgn) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* As = reinterpret_cast<double*>(smem_raw);      // 2 stages x {A [DM_KC][DM_LD], B [DM_KC][DM_LD]}
-    static_assert(sizeof(TA) == 8 && sizeof(TB) == 8, "FP64 operands");
-    const GemmTask t = tasks[blockIdx.x];
-    const int ldm = t.ldm;                        // rows of the whole output block and of A
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int wm = w % DM_WM, wn = w / DM_WM;
-    const int g = lane >> 2, tq = lane & 3;
-    double acc[DM_TI][DM_TJ][2];
-    #pragma unroll
-    for (int i = 0; i < DM_TI; ++i)
-        #pragma unroll
-        for (int j = 0; j < DM_TJ; ++j) { acc[i][j][0] = 0.0; acc[i][j][1] = 0.0; }
-    const int tm = (t.m + 7) >> 3, tn = (t.n + 7) >> 3;
-    // K is walked as one list of chunks over all pairs; chunk c+1 is copied
-    // into the other shared-memory stage (cp.async, zero-filled outside the
-    // operands) while chunk c feeds the tensor cores
-    int nchunk = 0;
-    for (int q = t.q_begin; q < t.q_end; ++q) nchunk += (pairs[q].k + DM_KC - 1) / DM_KC;
-    int lq = t.q_begin, lk0 = 0;                  // next chunk to load
-    auto issue = [&](int stage) {
-        const GemmPair pr = pairs[lq];
-        const TA* A = Abase + pr.a_off + t.r0;                  // the tile's rows of ldm x k, column-major
-        const TB* B = Bbase + pr.b_off + (int64_t)t.c0 * pr.k;  // the tile's columns of k x N, column-major
-        const int kc = min(DM_KC, pr.k - lk0);
-        double* as = As + stage * 2 * DM_KC * DM_LD;
-        double* bs = as + DM_KC * DM_LD;
-        for (int idx = threadIdx.x; idx < DM_KC * DM_MAX; idx += blockDim.x) {
-            const int i = idx % DM_MAX, kk = idx / DM_MAX;
-            const bool ok = i < t.m && kk < kc;
-            cp_async8(as + kk * DM_LD + i, ok ? (const void*)(A + i + (int64_t)(lk0 + kk) * ldm) : (const void*)A, ok);
-        }
-        for (int idx = threadIdx.x; idx < DM_KC * DM_MAX; idx += blockDim.x) {
-            const int kk = idx % DM_KC, j = idx / DM_KC;
-            const bool ok = j < t.n && kk < kc;
-            cp_async8(bs + kk * DM_LD + j, ok ? (const void*)(B + (lk0 + kk) + (int64_t)j * pr.k) : (const void*)B, ok);
-        }
-        cp_async_commit();
-        lk0 += DM_KC;
-        if (lk0 >= pr.k) { ++lq; lk0 = 0; }
-    };
-    int cq = t.q_begin, ck0 = 0;                  // chunk being computed
-    if (nchunk > 0) issue(0);
-    for (int c = 0; c < nchunk; ++c) {
-        if (c + 1 < nchunk) { issue((c + 1) & 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-        __syncthreads();
-        const int kc = min(DM_KC, pairs[cq].k - ck0);
-        const double* as = As + (c & 1) * 2 * DM_KC * DM_LD;
-        const double* bs = as + DM_KC * DM_LD;
-        for (int k8 = 0; k8 < kc; k8 += 8) {
-            // slices past kc read the stage's zeros (rows kc..31)
-            const double* a_lo = as + (k8 + tq) * DM_LD + g;       // A(., k8 + t)
-            const double* a_hi = a_lo + 4 * DM_LD;                 // A(., k8 + t + 4)
-            double b0[DM_TJ], b1[DM_TJ];
-            #pragma unroll
-            for (int j = 0; j < DM_TJ; ++j) {
-                // column tiles past the 17th exist only in the warp grid: never read them
-                const bool ok = wn + DM_WN * j < tn;
-                const int col = (wn + DM_WN * j) * 8 + g;
-                b0[j] = ok ? bs[(k8 + tq) * DM_LD + col] : 0.0;
-                b1[j] = ok ? bs[(k8 + tq + 4) * DM_LD + col] : 0.0;
-            }
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int p = wm + DM_WM * i;                      // rows 16p .. 16p + 15
-                if (2 * p >= tm) continue;
-                const double a0 = a_lo[16 * p], a1 = a_lo[16 * p + 8], a2 = a_hi[16 * p], a3 = a_hi[16 * p + 8];
-                #pragma unroll
-                for (int j = 0; j < DM_TJ; ++j) {
-                    if (wn + DM_WN * j >= tn) continue;
-                    dmma_16x8x8(acc[2 * i][j][0], acc[2 * i][j][1], acc[2 * i + 1][j][0], acc[2 * i + 1][j][1], a0, a1,
-                                a2, a3, b0[j], b1[j]);
-                }
-            }
-            if (wm == 0 && tm > 16) {                               // rows 128 .. 135
-                const double a0 = a_lo[128], a1 = a_hi[128];
-                #pragma unroll
-                for (int j = 0; j < DM_TJ; ++j) {
-                    if (wn + DM_WN * j >= tn) continue;
-                    dmma_8x8x4(acc[8][j][0], acc[8][j][1], a0, b0[j]);
-                    dmma_8x8x4(acc[8][j][0], acc[8][j][1], a1, b1[j]);
-                }
-            }
-        }
-        ck0 += DM_KC;
-        if (ck0 >= pairs[cq].k) { ++cq; ck0 = 0; }
-        __syncthreads();                          // stage (c & 1) is refilled two chunks later
-    }
-    // acc[2i + h]: rows 16 (wm + 2i) + 8h + g; acc[8] (warp row 0): rows 128 + g
-    #pragma unroll
-    for (int i = 0; i < DM_TI; ++i) {
-        const int row = (i < 8) ? 16 * (wm + DM_WM * (i >> 1)) + 8 * (i & 1) + g : (wm == 0 ? 128 + g : DM_MAX);
-        if (row >= t.m) continue;
-        #pragma unroll
-        for (int j = 0; j < DM_TJ; ++j) {
-            #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int col = (wn + DM_WN * j) * 8 + 2 * tq + e;
-                if (col >= t.n) continue;
-                const int64_t o = (t.r0 + row) + (int64_t)(t.c0 + col) * ldm;
-                double v = sgn * acc[i][j][e];
-                if (t.cinit_off >= 0) v = Cinit[t.cinit_off + o] + v;
-                Cbase[t.c_off + o] = from_d<TC>(v);
-            }
-        }
-    }
-}
-
 // FP32 SIMT version of the factor products for blocks up to 144 x 144, used
 // when the factors are only needed in FP32 (the mixed-precision inner solves):
 // one CTA per output block, 256 threads on a 16 x 16 grid, thread (tx, ty)
