@@ -375,6 +375,101 @@ __device__ __forceinline__ void face_node(const BoxGeom& g, const Tables& tb, co
     }
 }
 
+// ---- the blocks' contractions, on the FP64 tensor cores --------------------------
+// Block (f m, g n) = sum over the nodes k of A_g(f m, k) B(k, n): A the row
+// modes' (gradients') values times the pointwise derivative dF_f / dU_g, B the
+// column modes' values, the same for every g.  An item of a warp is row_tiles
+// tiles of 8 rows (f m, running over the fields without gaps: 135 rows are 17
+// tiles) by all five g and all modes n: up to 40 accumulator tiles of
+// mma.m8n8k4.  A lane forms its own entries of A in registers (one product,
+// or three for the volume's directions, feeding CT MMAs), so the derivative
+// data in shared memory is read once an item and the basis tables, through
+// L1, once for the five g.  The FP64 pipe bounds it: a slice of four nodes of
+// an order-2 item is 40 MMAs of 16 cycles against some 40 loads.
+__host__ __device__ constexpr int col_tiles(int nt) { return (nt + 7) / 8; }
+__host__ __device__ constexpr int row_tiles(int nt) { return col_tiles(nt) > 4 ? 1 : 2; }
+__host__ __device__ constexpr int row_items(int nt) { return ((5 * nt + 7) / 8 + row_tiles(nt) - 1) / row_tiles(nt); }
+
+template <int NT, int RT>
+__device__ __forceinline__ void clear_tiles(double (&acc)[RT][5][col_tiles(NT)][2]) {
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int gg = 0; gg < 5; ++gg)
+#pragma unroll
+            for (int j = 0; j < col_tiles(NT); ++j) { acc[i][gg][j][0] = 0.0; acc[i][gg][j][1] = 0.0; }
+}
+
+// acc += sum over nq nodes; rowtab [ND][nq][NT] (directions dstride apart),
+// coltab [nq][NT], w [nq][ND][5][5] (wq doubles a node); with directions the
+// volume term's sign
+template <int NT, int RT, int ND>
+__device__ __forceinline__ void contract(double (&acc)[RT][5][col_tiles(NT)][2], int nq, const double* __restrict__ rowtab,
+                                         size_t dstride, const double* __restrict__ coltab, const double* w, int wq, int rt0) {
+    constexpr int CT = col_tiles(NT);
+    const int lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
+    const double* rt[RT];
+    const double* wf[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+        const int row = min(8 * (rt0 + i) + g8, 5 * NT - 1);      // rows past the block repeat its last one and are not stored
+        rt[i] = rowtab + row % NT;
+        wf[i] = w + (row / NT) * 5;
+    }
+    const double* ct[CT];
+#pragma unroll
+    for (int j = 0; j < CT; ++j) ct[j] = coltab + min(8 * j + g8, NT - 1);
+#pragma unroll 1
+    for (int k0 = 0; k0 < nq; k0 += 4) {
+        const bool in = k0 + t4 < nq;
+        const int k = in ? k0 + t4 : nq - 1;
+        double bv[CT];
+#pragma unroll
+        for (int j = 0; j < CT; ++j) bv[j] = ct[j][k * NT];
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+            double gr[ND];
+#pragma unroll
+            for (int d = 0; d < ND; ++d) gr[d] = in ? rt[i][d * dstride + (size_t)k * NT] : 0.0;
+#pragma unroll
+            for (int gg = 0; gg < 5; ++gg) {
+                const double* wk = wf[i] + (size_t)k * wq + gg;
+                double a = gr[0] * wk[0];
+#pragma unroll
+                for (int d = 1; d < ND; ++d) a = fma(gr[d], wk[25 * d], a);
+                if (ND > 1) a = -a;
+#pragma unroll
+                for (int j = 0; j < CT; ++j) dmma_8x8x4(acc[i][gg][j][0], acc[i][gg][j][1], a, bv[j]);
+            }
+        }
+    }
+}
+
+// an item's tiles to (STORE) or from its rows of a column-major 5 NT x 5 NT block
+template <int NT, int RT, bool STORE>
+__device__ __forceinline__ void move_tiles(double (&acc)[RT][5][col_tiles(NT)][2], double* out, int rt0) {
+    const int lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+        const int row = 8 * (rt0 + i) + g8;
+#pragma unroll
+        for (int gg = 0; gg < 5; ++gg)
+#pragma unroll
+            for (int j = 0; j < col_tiles(NT); ++j)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int n = 8 * j + 2 * t4 + c;
+                    const bool ok = row < 5 * NT && n < NT;
+                    double* at = out + (int64_t)(gg * NT + n) * (5 * NT) + row;
+                    if (STORE) {
+                        if (ok) *at = acc[i][gg][j][c];
+                    } else {
+                        acc[i][gg][j][c] = ok ? *at : 0.0;
+                    }
+                }
+    }
+}
+
 // q and rhs: an element's segment at e * vs (vs = b for one time level, the
 // element's stride over all its levels under harmonic balance)
 template <int NT>
@@ -392,9 +487,26 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
     double* sFI = TWO ? sWF : sWdF + (size_t)qv * 75;   // [6][qf][5]
     double* sFs = sFI + (size_t)6 * qf * 5;     // [6][qf][5][5]  d integrand / d own state
     double* sFn = sFs + (size_t)6 * qf * 25;    // [6][qf][5][5]  d integrand / d neighbour state
-    int nbr[6];
+    constexpr int RT = row_tiles(NT), CT = col_tiles(NT), ITEMS = row_items(NT);
+    const int warp = threadIdx.x >> 5;
+    __shared__ int sFaces[6], sNext;            // faces with a neighbour; next item of the blocks
+    int nbr[6], nface = 0;
 #pragma unroll
-    for (int f = 0; f < 6; ++f) nbr[f] = neighbour(g, e, f);
+    for (int f = 0; f < 6; ++f) {
+        nbr[f] = neighbour(g, e, f);
+        if (nbr[f] >= 0) {
+            if (threadIdx.x == 0) sFaces[nface] = f;
+            ++nface;
+        }
+    }
+    if (threadIdx.x == 0) sNext = 0;
+    auto next_item = [&]() {
+        int it = 0;
+        if ((threadIdx.x & 31) == 0) it = atomicAdd(&sNext, 1);
+        return __shfl_sync(0xffffffffu, it, 0);
+    };
+    (void)warp;
+    (void)next_item;
 
     // 1. modes of the element and its neighbours
     for (int t = threadIdx.x; t < 7 * b; t += blockDim.x) {
@@ -429,86 +541,35 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
             rhs[(int64_t)e * vs + t] = r;
         }
 
-        // 4. DIAG block and 5. face blocks (skipped for a residual-only call): one
-        // thread per pair of (f, m, g) rows with the same f and g and modes m0,
-        // m0 + 1, all nt columns n of both in registers, so each basis value
-        // loaded feeds two FMAs; block entry (f nt + m, g nt + n) stored
-        // column-major.  Lanes of a warp take consecutive mode pairs.
+        // 4. DIAG block and face blocks (skipped for a residual-only call): the
+        // warps take items (a block, RT row tiles of it) as they come free,
+        // the DIAG block's, which are the long ones, first
         if (val == nullptr) return;
-        const int npair = (nt + 1) >> 1;
-        for (int blk = 6; blk >= 0; --blk) {
-            if (blk < 6 && nbr[blk] < 0) continue;
-            double* out = val + blk_off[(int64_t)e * 7 + blk];
-            for (int item = threadIdx.x; item < 25 * npair; item += blockDim.x) {
-                const int mp = item % npair, fg = item / npair, f = fg % 5, gg = fg / 5;
-                const int m0 = 2 * mp;
-                const bool two = m0 + 1 < nt;
-                const int m1 = two ? m0 + 1 : m0;
-                double a0[NT], a1[NT];
-#pragma unroll
-                for (int n = 0; n < NT; ++n) { a0[n] = 0.0; a1[n] = 0.0; }
-                if (blk == 6) {
-                    for (int qq = 0; qq < qv; ++qq) {
-                        const double w0 = sWdF[((qq * 3 + 0) * 5 + f) * 5 + gg];
-                        const double w1 = sWdF[((qq * 3 + 1) * 5 + f) * 5 + gg];
-                        const double w2 = sWdF[((qq * 3 + 2) * 5 + f) * 5 + gg];
-                        const double* g0 = tb.grad + (size_t)(0 * qv + qq) * nt;
-                        const double* g1 = tb.grad + (size_t)(1 * qv + qq) * nt;
-                        const double* g2 = tb.grad + (size_t)(2 * qv + qq) * nt;
-                        const double t0 = -(g0[m0] * w0 + g1[m0] * w1 + g2[m0] * w2);
-                        const double t1 = -(g0[m1] * w0 + g1[m1] * w1 + g2[m1] * w2);
-                        const double* ph = tb.phi + (size_t)qq * nt;
-#pragma unroll
-                        for (int n = 0; n < NT; ++n) {
-                            const double p = ph[n];
-                            a0[n] += t0 * p;
-                            a1[n] += t1 * p;
-                        }
-                    }
-                    for (int face = 0; face < 6; ++face) {
-                        for (int qq = 0; qq < qf; ++qq) {
-                            const double* pf = tb.phif + ((size_t)face * qf + qq) * nt;
-                            const double w = sFs[((size_t)face * qf + qq) * 25 + f * 5 + gg];
-                            const double t0 = pf[m0] * w, t1 = pf[m1] * w;
-#pragma unroll
-                            for (int n = 0; n < NT; ++n) {
-                                const double p = pf[n];
-                                a0[n] += t0 * p;
-                                a1[n] += t1 * p;
-                            }
-                        }
-                    }
-                } else {
-                    for (int qq = 0; qq < qf; ++qq) {
-                        const double* pf = tb.phif + ((size_t)blk * qf + qq) * nt;
-                        const double* pn = tb.phif + ((size_t)(blk ^ 1) * qf + qq) * nt;
-                        const double w = sFn[((size_t)blk * qf + qq) * 25 + f * 5 + gg];
-                        const double t0 = pf[m0] * w, t1 = pf[m1] * w;
-#pragma unroll
-                        for (int n = 0; n < NT; ++n) {
-                            const double p = pn[n];
-                            a0[n] += t0 * p;
-                            a1[n] += t1 * p;
-                        }
-                    }
+        const int* face_of = sFaces;
+        for (;;) {
+            const int it = next_item();
+            if (it >= (1 + nface) * ITEMS) break;
+            const int blk = it < ITEMS ? 6 : face_of[it / ITEMS - 1], rt0 = (it % ITEMS) * RT;
+            double acc[RT][5][CT][2];
+            clear_tiles<NT, RT>(acc);
+            if (blk == 6) {
+                contract<NT, RT, 3>(acc, qv, tb.grad, (size_t)qv * NT, tb.phi, sWdF, 75, rt0);
+                for (int face = 0; face < 6; ++face) {
+                    const double* pf = tb.phif + (size_t)face * qf * NT;
+                    contract<NT, RT, 1>(acc, qf, pf, 0, pf, sFs + (size_t)face * qf * 25, 25, rt0);
                 }
-                const int row = f * nt + m0;
-#pragma unroll
-                for (int n = 0; n < NT; ++n) {
-                    double* col = out + (int64_t)(gg * nt + n) * b + row;
-                    col[0] = a0[n];
-                    if (two) col[1] = a1[n];
-                }
+            } else {
+                contract<NT, RT, 1>(acc, qf, tb.phif + (size_t)blk * qf * NT, 0, tb.phif + (size_t)(blk ^ 1) * qf * NT,
+                                    sFn + (size_t)blk * qf * 25, 25, rt0);
             }
+            move_tiles<NT, RT, true>(acc, val + blk_off[(int64_t)e * 7 + blk], rt0);
         }
     } else {
         // Two passes over the same shared memory.  Every value is accumulated in
         // the single-pass order: the volume pass leaves the residual's and the
         // DIAG block's volume sums in the outputs, and the face pass reloads and
         // continues them (each output value is read back by the thread that
-        // wrote it).  Block rows: one (f, m, g) row and one half of its nt
-        // columns per item, so the accumulators fit in registers.
-        constexpr int NH = NT / 2;
+        // wrote it).
         const int64_t* bo = blk_off + (int64_t)e * 7;
         // ---- volume pass
         for (int t = threadIdx.x; t < qv; t += blockDim.x) volume_node<NT>(tb, sU, t, nt, sWF, sWdF);
@@ -522,28 +583,13 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
                    + tb.grad[(2 * qv + qq) * nt + m] * sWF[(qq * 3 + 2) * 5 + f];
             rhs[(int64_t)e * vs + t] = r;
         }
-        if (val != nullptr) {
-            double* out = val + bo[6];
-            for (int item = threadIdx.x; item < 25 * nt * 2; item += blockDim.x) {
-                const int h = item & 1, m = (item >> 1) % nt, fg = (item >> 1) / nt, f = fg % 5, gg = fg / 5;
-                double a0[NH];
-#pragma unroll
-                for (int n = 0; n < NH; ++n) a0[n] = 0.0;
-                for (int qq = 0; qq < qv; ++qq) {
-                    const double w0 = sWdF[((qq * 3 + 0) * 5 + f) * 5 + gg];
-                    const double w1 = sWdF[((qq * 3 + 1) * 5 + f) * 5 + gg];
-                    const double w2 = sWdF[((qq * 3 + 2) * 5 + f) * 5 + gg];
-                    const double t0 = -(tb.grad[(size_t)(0 * qv + qq) * nt + m] * w0 +
-                                        tb.grad[(size_t)(1 * qv + qq) * nt + m] * w1 +
-                                        tb.grad[(size_t)(2 * qv + qq) * nt + m] * w2);
-                    const double* ph = tb.phi + (size_t)qq * nt + h * NH;
-#pragma unroll
-                    for (int n = 0; n < NH; ++n) a0[n] += t0 * ph[n];
-                }
-#pragma unroll
-                for (int n = 0; n < NH; ++n) out[(int64_t)(gg * nt + h * NH + n) * b + f * nt + m] = a0[n];
+        if (val != nullptr)
+            for (int rt = warp; rt < ITEMS; rt += kThreads / 32) {
+                double acc[RT][5][CT][2];
+                clear_tiles<NT, RT>(acc);
+                contract<NT, RT, 3>(acc, qv, tb.grad, (size_t)qv * NT, tb.phi, sWdF, 75, rt * RT);
+                move_tiles<NT, RT, true>(acc, val + bo[6], rt * RT);
             }
-        }
         __syncthreads();
         // ---- face pass
         for (int t = threadIdx.x; t < 6 * qf; t += blockDim.x) {
@@ -560,37 +606,22 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
             rhs[(int64_t)e * vs + t] = r;
         }
         if (val == nullptr) return;
-        for (int blk = 6; blk >= 0; --blk) {
-            if (blk < 6 && nbr[blk] < 0) continue;
-            double* out = val + bo[blk];
-            for (int item = threadIdx.x; item < 25 * nt * 2; item += blockDim.x) {
-                const int h = item & 1, m = (item >> 1) % nt, fg = (item >> 1) / nt, f = fg % 5, gg = fg / 5;
-                double a0[NH];
-                double* dst = out + (int64_t)(gg * nt + h * NH) * b + f * nt + m;
-                if (blk == 6) {
-#pragma unroll
-                    for (int n = 0; n < NH; ++n) a0[n] = dst[(int64_t)n * b];
-                    for (int face = 0; face < 6; ++face)
-                        for (int qq = 0; qq < qf; ++qq) {
-                            const double* pf = tb.phif + ((size_t)face * qf + qq) * nt;
-                            const double t0 = pf[m] * sFs[((size_t)face * qf + qq) * 25 + f * 5 + gg];
-#pragma unroll
-                            for (int n = 0; n < NH; ++n) a0[n] += t0 * pf[h * NH + n];
-                        }
-                } else {
-#pragma unroll
-                    for (int n = 0; n < NH; ++n) a0[n] = 0.0;
-                    for (int qq = 0; qq < qf; ++qq) {
-                        const double* pf = tb.phif + ((size_t)blk * qf + qq) * nt;
-                        const double* pn = tb.phif + ((size_t)(blk ^ 1) * qf + qq) * nt + h * NH;
-                        const double t0 = pf[m] * sFn[((size_t)blk * qf + qq) * 25 + f * 5 + gg];
-#pragma unroll
-                        for (int n = 0; n < NH; ++n) a0[n] += t0 * pn[n];
-                    }
+        // the DIAG block's items on the warps that stored their volume sums
+        for (int it = warp; it < (1 + nface) * ITEMS; it += kThreads / 32) {
+            const int blk = it < ITEMS ? 6 : sFaces[it / ITEMS - 1], rt0 = (it % ITEMS) * RT;
+            double acc[RT][5][CT][2];
+            if (blk == 6) {
+                move_tiles<NT, RT, false>(acc, val + bo[6], rt0);
+                for (int face = 0; face < 6; ++face) {
+                    const double* pf = tb.phif + (size_t)face * qf * NT;
+                    contract<NT, RT, 1>(acc, qf, pf, 0, pf, sFs + (size_t)face * qf * 25, 25, rt0);
                 }
-#pragma unroll
-                for (int n = 0; n < NH; ++n) dst[(int64_t)n * b] = a0[n];
+            } else {
+                clear_tiles<NT, RT>(acc);
+                contract<NT, RT, 1>(acc, qf, tb.phif + (size_t)blk * qf * NT, 0, tb.phif + (size_t)(blk ^ 1) * qf * NT,
+                                    sFn + (size_t)blk * qf * 25, 25, rt0);
             }
+            move_tiles<NT, RT, true>(acc, val + bo[blk], rt0);
         }
     }
 }
