@@ -182,20 +182,22 @@ int chidg::push_scalars(chidg_gpu_ctx* ctx, int slot, int count, const double* i
     return CHIDG_GPU_OK;
 }
 
+unsigned* chidg::cta_counter(chidg_gpu_ctx* ctx) { return (unsigned*)ctx->d_status + 2; }
+
 // dot products of x with nq vectors y + q*ystride, results in d_scal[slot+q]
 template <typename T>
-int chidg::mdot(chidg_gpu_ctx* ctx, int64_t n, const T* x, const T* y, int64_t ystride, int nq, int slot) {
+int chidg::mdot(chidg_gpu_ctx* ctx, int64_t n, const T* x, const T* y, int64_t ystride, int nq, int slot, const double* rows,
+                int nrow, int row_slot) {
     const int threads = 256;
     const int ncta = grid_for(n, threads, ctx->nsm * 4);
-    int st = ensure(ctx, ctx->partial, sizeof(double) * (size_t)ncta * std::max(nq, 1));
+    int st = ensure(ctx, ctx->partial, sizeof(double) * (size_t)ncta * (std::max(nq, 1) + 1));
     if (st) return st;
-    k_mdot_partial<T><<<ncta, threads, 0, ctx->stream>>>(n, x, y, ystride, nq, (double*)ctx->partial.ptr);
-    st = check_launch(ctx, "k_mdot_partial");
-    if (st) return st;
-    return reduce_partials(ctx, (const double*)ctx->partial.ptr, ncta, nq, slot, false);
+    k_mdot<T><<<ncta, threads, 0, ctx->stream>>>(n, x, y, ystride, nq, (double*)ctx->partial.ptr, ctx->d_scal + slot, rows,
+                                                nrow, ctx->d_scal + row_slot, cta_counter(ctx));
+    return check_launch(ctx, "k_mdot");
 }
-template int chidg::mdot<double>(chidg_gpu_ctx*, int64_t, const double*, const double*, int64_t, int, int);
-template int chidg::mdot<float>(chidg_gpu_ctx*, int64_t, const float*, const float*, int64_t, int, int);
+template int chidg::mdot<double>(chidg_gpu_ctx*, int64_t, const double*, const double*, int64_t, int, int, const double*, int, int);
+template int chidg::mdot<float>(chidg_gpu_ctx*, int64_t, const float*, const float*, int64_t, int, int, const double*, int, int);
 
 extern "C" int chidg_gpu_ctx_create(int device, void* stream, chidg_gpu_ctx** out) {
     if (!out) return CHIDG_GPU_EINVAL;
@@ -221,6 +223,12 @@ extern "C" int chidg_gpu_ctx_create(int device, void* stream, chidg_gpu_ctx** ou
         cudaGetLastError();
         chidg_gpu_ctx_destroy(ctx);
         return CHIDG_GPU_ENOMEM;
+    }
+    // the CTA counter starts at zero (on the stream that uses it)
+    if (cudaMemsetAsync(ctx->d_status, 0, sizeof(int) * 4, ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        chidg_gpu_ctx_destroy(ctx);
+        return CHIDG_GPU_ECUDA;
     }
     *out = ctx;
     return CHIDG_GPU_OK;

@@ -32,6 +32,7 @@ constexpr int kSlotWnorm = 2;      // ||w||^2 after orthogonalisation
 constexpr int kSlotR0 = 3;         // ||r0||^2
 constexpr int kSlotStatus = 4;     // int status word of the dataflow sweeps (nonzero = a wait ran out)
 constexpr long long kSpinLimit = 2000000000LL;   // clock cycles a sweep waits for a parent (~1 s)
+constexpr int kSlotReorth = 5;     // 1: the last Gram-Schmidt pass asks for a second one
 constexpr int kSlotH = 16;         // h(1:j, j) of the current pass (up to 4000 entries)
 constexpr int kSlotY = 4096;       // y coefficients of the solution update (up to 4000 entries)
 constexpr int kSlotFields = 8160;  // per-field norms (up to 32 fields)
@@ -229,8 +230,12 @@ int grid_for(int64_t n, int threads, int cap);
 int reduce_partials(chidg_gpu_ctx* ctx, const double* partial, int ncta, int nq, int slot, bool do_sqrt);
 int fetch_scalars(chidg_gpu_ctx* ctx, int slot, int count, double* out);
 int push_scalars(chidg_gpu_ctx* ctx, int slot, int count, const double* in);
+// dot products of x with nq vectors into d_scal[slot..]; with rows also
+// d_scal[row_slot] = sum of rows[0..nrow)
 template <typename T>
-int mdot(chidg_gpu_ctx* ctx, int64_t n, const T* x, const T* y, int64_t ystride, int nq, int slot);
+int mdot(chidg_gpu_ctx* ctx, int64_t n, const T* x, const T* y, int64_t ystride, int nq, int slot,
+         const double* rows = nullptr, int nrow = 0, int row_slot = 0);
+unsigned* cta_counter(chidg_gpu_ctx* ctx);      // zero between launches (last_cta)
 int matrix_lowp(chidg_gpu_matrix* A, int precision);
 // The matrix the operators act on: A itself, or A^T (A->T, its values
 // re-transposed when A's stamp changed) when A->transposed is set.

@@ -110,26 +110,34 @@ struct Solver {
         k_axpby<T, T><<<grid_for(n, 256, ctx->nsm * 8), 256, 0, ctx->stream>>>(n, a, nullptr, x, b, y);
         return check_launch(ctx, "k_axpby");
     }
-    // one Gram-Schmidt pass; h(0:j) for this pass left in d_scal[kSlotH..], ||w||^2 in kSlotWnorm
-    int gs_pass(T* w, const T* Vb, int j) {
+    // one Gram-Schmidt pass; h(0:j) for this pass left in d_scal[kSlotH..], ||w||^2 in kSlotWnorm.
+    // With rows (w's row sums of squares) also ||w||^2 before the pass in
+    // kSlotNormBefore and whether a second pass is due in kSlotReorth.
+    int gs_pass(T* w, const T* Vb, int j, const double* rows = nullptr) {
         const int64_t n = A->n;
         int st;
         const int threads = 256;
         const int ncta = grid_for(n, threads, ctx->nsm * 4);
         if ((st = ensure(ctx, ctx->partial2, sizeof(double) * (size_t)ncta))) return st;
+        double* sc = ctx->d_scal;
+        double* pt = (double*)ctx->partial2.ptr;
+        const double* before = rows ? sc + kSlotNormBefore : nullptr;
         if (orth == CHIDG_ORTH_CGS) {
-            if ((st = mdot<T>(ctx, n, w, Vb, n, j, kSlotH))) return st;
-            k_maxpy_sub_norm<T><<<ncta, threads, 0, ctx->stream>>>(n, w, Vb, n, j, ctx->d_scal + kSlotH, (double*)ctx->partial2.ptr);
-            if ((st = check_launch(ctx, "k_maxpy_sub_norm"))) return st;
-        } else {
-            for (int i = 0; i < j; ++i) {
-                if ((st = mdot<T>(ctx, n, w, Vb + (int64_t)i * n, n, 1, kSlotH + i))) return st;
-                k_maxpy_sub_norm<T><<<ncta, threads, 0, ctx->stream>>>(n, w, Vb + (int64_t)i * n, n, 1, ctx->d_scal + kSlotH + i,
-                                                                       (i == j - 1) ? (double*)ctx->partial2.ptr : nullptr);
-                if ((st = check_launch(ctx, "k_maxpy_sub_norm"))) return st;
-            }
+            if ((st = mdot<T>(ctx, n, w, Vb, n, j, kSlotH, rows, A->nrow, kSlotNormBefore))) return st;
+            k_maxpy_sub_norm<T><<<ncta, threads, 0, ctx->stream>>>(n, w, Vb, n, j, sc + kSlotH, pt, sc + kSlotWnorm, before,
+                                                                   sc + kSlotReorth, cta_counter(ctx));
+            return check_launch(ctx, "k_maxpy_sub_norm");
         }
-        return reduce_partials(ctx, (const double*)ctx->partial2.ptr, ncta, 1, kSlotWnorm, false);
+        for (int i = 0; i < j; ++i) {
+            if ((st = mdot<T>(ctx, n, w, Vb + (int64_t)i * n, n, 1, kSlotH + i, i == 0 ? rows : nullptr, A->nrow, kSlotNormBefore)))
+                return st;
+            const bool last = i == j - 1;
+            k_maxpy_sub_norm<T><<<ncta, threads, 0, ctx->stream>>>(n, w, Vb + (int64_t)i * n, n, 1, sc + kSlotH + i,
+                                                                   last ? pt : nullptr, sc + kSlotWnorm, nullptr, nullptr,
+                                                                   cta_counter(ctx));
+            if ((st = check_launch(ctx, "k_maxpy_sub_norm"))) return st;
+        }
+        return CHIDG_GPU_OK;
     }
 
     int solve(const T* b, T* x) {
@@ -190,13 +198,8 @@ struct Solver {
                 if (precon_mv && !inner) {
                     if ((st = ensure(ctx, ws->rowsq, sizeof(double) * (size_t)A->nrow))) return st;
                     st = precon_mv(vj, zj, w, (double*)ws->rowsq.ptr);
-                    if (st == CHIDG_GPU_OK) {
-                        fused = true;
-                        if ((st = reduce_partials(ctx, (const double*)ws->rowsq.ptr, A->nrow, 1, kSlotNormBefore, false)))
-                            return st;
-                    } else if (st != 1) {
-                        return st;
-                    }
+                    if (st == CHIDG_GPU_OK) fused = true;
+                    else if (st != 1) return st;
                 }
                 if (!fused) {
                     if ((st = precon(vj, zj))) return st;
@@ -208,9 +211,19 @@ struct Solver {
                         inner_iters += child->niter;
                         if ((st = axpby(1.0, DZ, 1.0, zj))) return st;                     // z = z + dz
                     }
-                    if ((st = matvec(zj, w, nullptr, 1.0, 0.0, true, kSlotNormBefore))) return st;
+                    if ((st = ensure(ctx, ws->rowsq, sizeof(double) * (size_t)A->nrow)) ||
+                        (st = launch_mv(zj, w, nullptr, 1.0, 0.0, (double*)ws->rowsq.ptr)))
+                        return st;
                 }
-                if ((st = gs_pass(w, Vb, j))) return st;
+                // the projections, and v(j+1) = w / h(j+1,j) unless a second pass
+                // is due (decided on the device: nothing waits for the host here)
+                const bool cgs = orth == CHIDG_ORTH_CGS;
+                if ((st = gs_pass(w, Vb, j, (const double*)ws->rowsq.ptr))) return st;
+                if (cgs) {
+                    k_scale_next<T><<<grid_for(n, 256, ctx->nsm * 8), 256, 0, ctx->stream>>>(n, w, ctx->d_scal + kSlotWnorm,
+                                                                                             ctx->d_scal + kSlotReorth);
+                    if ((st = check_launch(ctx, "k_scale_next"))) return st;
+                }
                 if ((st = fetch_scalars(ctx, 0, kSlotH + j, sc.data()))) return st;
                 if ((st = status_word(ctx, sc[kSlotStatus]))) return st;
                 const double norm_before = std::sqrt(sc[kSlotNormBefore]);
@@ -218,10 +231,13 @@ struct Solver {
                 std::vector<double> hcol(sc.begin() + kSlotH, sc.begin() + kSlotH + j);
                 double wn2 = sc[kSlotWnorm];
                 // selective re-orthogonalisation (:203-223)
-                double crit = 0.0;
-                for (int i = 0; i < j; ++i) crit += std::fabs(hcol[i]);
-                crit /= norm_before;
-                if (crit >= 1.0) {
+                bool again = sc[kSlotReorth] != 0.0;
+                if (!cgs) {
+                    double crit = 0.0;
+                    for (int i = 0; i < j; ++i) crit += std::fabs(hcol[i]);
+                    again = crit / norm_before >= 1.0;
+                }
+                if (again) {
                     if ((st = gs_pass(w, Vb, j))) return st;
                     if ((st = fetch_scalars(ctx, 0, kSlotH + j, sc.data()))) return st;
                     for (int i = 0; i < j; ++i) hcol[i] += sc[kSlotH + i];
@@ -229,7 +245,8 @@ struct Solver {
                 }
                 for (int i = 0; i < j; ++i) H(i, j - 1) = hcol[i];
                 H(j, j - 1) = std::sqrt(wn2);
-                if ((st = axpby(1.0 / H(j, j - 1), w, 0.0, w))) return st;   // v(j+1) = w / h(j+1,j)
+                if (!cgs || again)                                           // v(j+1) = w / h(j+1,j)
+                    if ((st = axpby(1.0 / H(j, j - 1), w, 0.0, w))) return st;
                 for (int i = 0; i < j - 1; ++i) {
                     const double hij = c[i] * H(i, j - 1) + s[i] * H(i + 1, j - 1);
                     const double hipj = -s[i] * H(i, j - 1) + c[i] * H(i + 1, j - 1);

@@ -176,10 +176,42 @@ __global__ void __launch_bounds__(1024) k_matvec(const TA* __restrict__ val, con
 // BLAS-1.  All reductions are two-pass: per-CTA partials in fixed order, then
 // one CTA sums the partials in fixed order, so results are reproducible.
 // ---------------------------------------------------------------------------
-// partial[q * gridDim.x + blockIdx.x] = sum_i x[i] * y_q[i],  y_q = y + q * ystride
+// True in every thread of the last CTA of the launch to get here (the writes
+// of the others are then visible); the counter is left at zero.
+__device__ __forceinline__ bool last_cta(unsigned* counter) {
+    __shared__ unsigned s_ticket;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_ticket = atomicAdd(counter, 1u);
+    __syncthreads();
+    if (s_ticket != gridDim.x - 1) return false;
+    if (threadIdx.x == 0) *counter = 0u;
+    __threadfence();
+    return true;
+}
+// out[q] = sum_c partial[q * ncta + c], q < nq: a warp a sum, in a fixed order
+__device__ __forceinline__ void sum_partials(const double* partial, int ncta, int nq, double* out) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int q = threadIdx.x >> 5; q < nq; q += nw) {
+        double s = 0.0;
+        #pragma unroll 4
+        for (int c = lane; c < ncta; c += 32) s += __ldcg(partial + (int64_t)q * ncta + c);
+        s = warp_sum(s);
+        if (lane == 0) out[q] = s;
+    }
+}
+// out[q] = sum_i x[i] * y_q[i], y_q = y + q * ystride, q < nq, and, with rows,
+// row_out = sum_r rows[r] (the row sums of squares of the product before): the
+// CTAs leave partial[q * gridDim.x + blockIdx.x], the last one adds them up, so
+// the sums of a Gram-Schmidt pass are one launch.  (A reduction launch of its
+// own, one CTA taking the sums one after another, was 11 us a pass at 30
+// vectors.  An Arnoldi step of a 6 x 7 x 5 harmonic-balance box of order 1
+// takes 12 us less with the three reductions inside the passes and the scaling
+// not waiting for the host.)
 template <typename T>
-__global__ void k_mdot_partial(int64_t n, const T* __restrict__ x, const T* __restrict__ y,
-                               int64_t ystride, int nq, double* __restrict__ partial) {
+__global__ void k_mdot(int64_t n, const T* __restrict__ x, const T* __restrict__ y, int64_t ystride, int nq,
+                       double* __restrict__ partial, double* out, const double* __restrict__ rows, int nrow,
+                       double* row_out, unsigned* counter) {
     // eight vectors per pass over x: x[i] is read once for the eight, and the
     // eight loads of y are in flight together; each sum is formed in the
     // order of a pass per vector (thread's i in stride order, then the
@@ -187,6 +219,13 @@ __global__ void k_mdot_partial(int64_t n, const T* __restrict__ x, const T* __re
     constexpr int QG = 8;
     __shared__ double scratch[QG][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (rows != nullptr) {
+        double s = 0.0;
+        for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrow; r += gridDim.x * blockDim.x) s += rows[r];
+        s = block_sum(s, scratch[0]);
+        if (threadIdx.x == 0) partial[(int64_t)nq * gridDim.x + blockIdx.x] = s;
+        __syncthreads();
+    }
     for (int q0 = 0; q0 < nq; q0 += QG) {
         const int qn = min(QG, nq - q0);
         const T* yq = y + (int64_t)q0 * ystride;
@@ -217,6 +256,9 @@ __global__ void k_mdot_partial(int64_t n, const T* __restrict__ x, const T* __re
             }
         }
     }
+    if (!last_cta(counter)) return;
+    sum_partials(partial, gridDim.x, nq, out);
+    if (rows != nullptr) sum_partials(partial + (int64_t)nq * gridDim.x, gridDim.x, 1, row_out);
 }
 // out[q] = sum_c partial[q * ncta + c]  (optionally sqrt)
 static __global__ void k_reduce_partials(const double* __restrict__ partial, int ncta, int nq,
@@ -250,10 +292,15 @@ static __global__ void k_field_sumsq(const double* __restrict__ x, const int64_t
         __syncthreads();
     }
 }
-// w[i] = w[i] - sum_q h[q] * v_q[i]  (CGS update, h on device), with sum of squares partials
+// w[i] = w[i] - sum_q h[q] * v_q[i]  (CGS update, h on device).  With partial,
+// norm2[0] = |w|^2 of the result (the last CTA adds the CTAs' sums up) and, with
+// before2 (|w|^2 before the pass), reorth[0] = 1 if sum |h| / |w before| >= 1
+// (the selective second pass, type_fgmres.f90:203-223), 0 otherwise: a vector
+// that needs no second pass can be scaled without asking the host.
 template <typename T>
 __global__ void k_maxpy_sub_norm(int64_t n, T* __restrict__ w, const T* __restrict__ v, int64_t vstride,
-                                 int nq, const double* __restrict__ h, double* __restrict__ partial) {
+                                 int nq, const double* __restrict__ h, double* __restrict__ partial, double* norm2,
+                                 const double* __restrict__ before2, double* reorth, unsigned* counter) {
     __shared__ double scratch[32];
     __shared__ double hs[128];
     double sq = 0.0;
@@ -271,10 +318,24 @@ __global__ void k_maxpy_sub_norm(int64_t n, T* __restrict__ w, const T* __restri
             if (last) { const double od = to_d(o); sq += od * od; }
         }
     }
-    if (partial != nullptr) {
-        sq = block_sum(sq, scratch);
-        if (threadIdx.x == 0) partial[blockIdx.x] = sq;
+    if (partial == nullptr) return;
+    sq = block_sum(sq, scratch);
+    if (threadIdx.x == 0) partial[blockIdx.x] = sq;
+    if (!last_cta(counter)) return;
+    sum_partials(partial, gridDim.x, 1, norm2);
+    if (before2 != nullptr && threadIdx.x == 32) {
+        double crit = 0.0;
+        for (int q = 0; q < nq; ++q) crit += fabs(h[q]);
+        reorth[0] = crit / sqrt(before2[0]) >= 1.0 ? 1.0 : 0.0;
     }
+}
+// v = w / sqrt(norm2[0]) in place, unless skip[0] is set
+template <typename T>
+__global__ void k_scale_next(int64_t n, T* w, const double* norm2, const double* skip) {
+    if (skip[0] != 0.0) return;
+    const double a = 1.0 / sqrt(norm2[0]);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        w[i] = from_d<T>(a * to_d(w[i]));
 }
 // MGS single step: w -= h[0] * v (h on device), with sum-of-squares partials
 // x = x0 + sum_q y[q] * z_q   (y on device)
