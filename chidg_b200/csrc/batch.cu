@@ -714,7 +714,6 @@ extern "C" int chidg_gpu_fgmres_solve_batched(chidg_gpu_matrix* A, chidg_gpu_pre
     if ((st = matrix_op(A, &A))) return st;
     // the FP32 / BF16 copy read by the inner solves' products
     if (inner && (st = matrix_lowp(A, prec))) return st;
-    set_matvec_smem(A);
     if (M->kind != CHIDG_PRECON_IDENTITY) precon_set_smem(M);
     cudaMemsetAsync(ctx->d_scal + kSlotStatus, 0, sizeof(double), ctx->stream);
 

@@ -429,6 +429,16 @@ extern "C" int chidg_gpu_matrix_create(chidg_gpu_ctx* ctx, const chidg_gpu_patte
         chidg_gpu_matrix_destroy(A);
         return st;
     }
+    if (*std::min_element(rb.begin(), rb.end()) != A->max_b) {
+        // rows by falling cost, for the streamed matvec
+        std::vector<int64_t> cost(A->nrow);
+        for (int r = 0; r < A->nrow; ++r)
+            for (int32_t k : A->rowblk[r]) cost[r] += (int64_t)rb[r] * A->bsize(A->ce[k]);
+        std::vector<int32_t> order(A->nrow);
+        for (int r = 0; r < A->nrow; ++r) order[r] = r;
+        std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
+        if ((st = upload_array(ctx, A->d_row_order, order))) { chidg_gpu_matrix_destroy(A); return st; }
+    }
     if ((st = ensure(ctx, A->val, sizeof(double) * (size_t)A->nval))) { chidg_gpu_matrix_destroy(A); return st; }
     cudaMemsetAsync(A->val.ptr, 0, sizeof(double) * (size_t)A->nval, ctx->stream);
     A->mv_threads = launch_dim_for(MV_GCAP, rb);
@@ -443,7 +453,7 @@ extern "C" int chidg_gpu_matrix_destroy(chidg_gpu_matrix* A) {
     cudaStreamSynchronize(A->ctx->stream);
     for (Buffer* b : {&A->val, &A->val32, &A->val16, &A->d_row_ptr, &A->d_blk_voff, &A->d_blk_xoff, &A->d_blk_nc,
                       &A->d_row_yoff, &A->d_row_b, &A->d_diag_voff, &A->d_elem_nvars, &A->d_elem_nterms, &A->row_sq,
-                      &A->d_tr_src, &A->d_tr_dst, &A->d_tr_nr, &A->d_tr_nc, &A->d_mass_off, &A->d_scale_off})
+                      &A->d_tr_src, &A->d_tr_dst, &A->d_tr_nr, &A->d_tr_nc, &A->d_mass_off, &A->d_scale_off, &A->d_row_order})
         release(*b);
     if (A->T) chidg_gpu_matrix_destroy(A->T);
     delete A;
@@ -761,7 +771,7 @@ int chidg::matvec_launch(chidg_gpu_matrix* A, const TA* val, const TV* x, TV* y,
             const RowMask mk = ctx->row_mask.nrow == A->nrow ? ctx->row_mask : RowMask{};
             k<<<grid, 32 * cw + 32, smem, ctx->stream>>>(R, A->nrow, val, x, y, z, alpha, beta, row_sq,
                                                          (int*)(ctx->d_scal + kSlotStatus), kSpinLimit, sh.nstage,
-                                                         sh.stage_bytes, A->max_row_cols, mk);
+                                                         sh.stage_bytes, A->max_row_cols, mk, (const int32_t*)A->d_row_order.ptr);
             return CHIDG_GPU_OK;
         };
         int st2;
@@ -773,6 +783,8 @@ int chidg::matvec_launch(chidg_gpu_matrix* A, const TA* val, const TV* x, TV* y,
         if (st2) return st2;
     } else {
         const size_t smem = sizeof(ACC) * ((size_t)A->max_row_cols + A->mv_threads) + 512;
+        const int st2 = set_matvec_smem(A);
+        if (st2) return fail(ctx, st2, "matvec shared memory");
         k_matvec<TA, TV, TV, ACC><<<A->nrow, A->mv_threads, smem, ctx->stream>>>(
             val, (const int64_t*)A->d_row_ptr.ptr, (const int64_t*)A->d_blk_voff.ptr, (const int64_t*)A->d_blk_xoff.ptr,
             (const int32_t*)A->d_blk_nc.ptr, (const int64_t*)A->d_row_yoff.ptr, (const int32_t*)A->d_row_b.ptr, x, y, z, alpha, beta, row_sq);
@@ -985,7 +997,6 @@ extern "C" int chidg_gpu_matvec(chidg_gpu_matrix* A, const chidg_gpu_vector* x, 
     chidg_gpu_matrix* S;                 // A, or A^T when A->transposed (operator_chidg_mv.f90:46-60)
     int st = matrix_op(A, &S);
     if (st) return st;
-    set_matvec_smem(S);
     return matvec_launch<double, double>(S, (const double*)S->val.ptr, (const double*)x->buf.ptr, (double*)y->buf.ptr,
                                          nullptr, 1.0, 0.0, nullptr);
 }
@@ -2684,7 +2695,6 @@ extern "C" int chidg_gpu_autotune(chidg_gpu_precon* M, chidg_gpu_matrix* A, int3
     int st;
     if ((st = matrix_op(A, &Aop))) return st;
     if ((st = matrix_lowp(Aop, precision))) return st;
-    set_matvec_smem(Aop);
     precon_set_smem(M);
     const bool lowp_vec = precision == CHIDG_GPU_MIXED_FP32 || precision == CHIDG_GPU_MIXED_BF16;
     const int esz_blocks = precision == CHIDG_GPU_FP64 ? 8 : precision == CHIDG_GPU_MIXED_BF16 ? 2 : 4;

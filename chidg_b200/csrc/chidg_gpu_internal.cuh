@@ -176,7 +176,7 @@ struct chidg_gpu_matrix {
     chidg::Buffer val, val32, val16;
     int64_t val32_stamp = -1, val16_stamp = -1;
     chidg::Buffer d_row_ptr, d_blk_voff, d_blk_xoff, d_blk_nc, d_row_yoff, d_row_b, d_diag_voff, d_elem_nvars,
-        d_elem_nterms, row_sq;
+        d_elem_nterms, row_sq, d_row_order;   // d_row_order: rows by falling size (several block sizes only)
     int64_t stamp = 0;
     // chidg_matrix_t%transposed (type_chidg_matrix.f90:49): products, ILU0 and
     // Jacobi then act on A^T, kept as a second matrix T in block-row storage

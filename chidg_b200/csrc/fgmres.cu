@@ -354,7 +354,6 @@ extern "C" int chidg_gpu_fgmres_solve(chidg_gpu_matrix* A, chidg_gpu_precon* M, 
     if ((o.precision == CHIDG_GPU_MIXED_FP32 || o.precision == CHIDG_GPU_MIXED_BF16) &&
         (st = matrix_lowp(Aop, o.precision)))
         return st;
-    set_matvec_smem(Aop);
     if (M->kind != CHIDG_PRECON_IDENTITY) precon_set_smem(M);
     ctx->err_elem = -1;
     cudaMemsetAsync(ctx->d_scal + kSlotStatus, 0, sizeof(double), ctx->stream);

@@ -4,8 +4,11 @@
 // A row's blocks are stored one after another, all with the row's b rows, so
 // the row is one column-major b x ncols matrix (ncols = sum of the blocks'
 // columns) and its x segments, concatenated, are the vector it multiplies.
-// Persistent CTAs: a producer lane takes rows blockIdx.x, blockIdx.x + gridDim.x,
-// ... (rows are alike in size) and copies each row's
+// Persistent CTAs: a producer lane takes the rows at positions blockIdx.x,
+// blockIdx.x + gridDim.x, ... of `order` (null: as they stand; a matrix of
+// several block sizes lists its rows by falling size, so that every turn hands
+// the CTAs rows of alike cost and the last turns are short: 11 x 13 x 12
+// elements of orders 1 to 3 take 457 us, 583 us in natural order) and copies each row's
 // values, in column chunks, into a ring of shared-memory stages with
 // cp.async.bulk (source rounded to 16 bytes, as in the streamed sweeps); the
 // consumer warps stage the row's x segments, multiply the chunks as they land
@@ -35,7 +38,7 @@ __global__ void __launch_bounds__(32 * CW + 32)
     k_matvec_stream(MatvecRows R, int nrow, const TA* __restrict__ val, const TX* __restrict__ x, TX* __restrict__ y,
                     const TX* __restrict__ z, double alpha, double beta, double* __restrict__ row_sumsq,
                     int* __restrict__ status, long long spin_limit, int nstage,
-                    int stage_bytes, int max_cols, RowMask mask) {
+                    int stage_bytes, int max_cols, RowMask mask, const int32_t* __restrict__ order) {
     constexpr int NC = 32 * CW;
     constexpr int RPT = (SS_MAX_B + NC - 1) / NC;
     extern __shared__ __align__(128) unsigned char ss_smem[];
@@ -63,8 +66,9 @@ __global__ void __launch_bounds__(32 * CW + 32)
         if (lane != 0) return;
         int stage = 0;
         unsigned phase = 0;
-        for (int row = blockIdx.x;; row += gridDim.x) {
-            if (row >= nrow) {
+        for (int pos = blockIdx.x;; pos += gridDim.x) {
+            const int row = pos < nrow && order != nullptr ? order[pos] : pos;
+            if (pos >= nrow) {
                 if (!mbar_wait(empty + stage, phase ^ 1u, spin_limit)) atomicExch(status, 1);
                 meta[stage].task = -1;
                 mbar_arrive(full + stage);
