@@ -1263,13 +1263,9 @@ static int build_rasilu0(const chidg_gpu_matrix* A, IluProgram& P, std::string& 
     return CHIDG_GPU_OK;
 }
 
-// Register-tile class of the diagonal-block inverse for block size b.
-// inverse kernel by block size: 0..1 register-tiled Gauss-Jordan (b <= 64),
-// 2 tensor-core blocked Gauss-Jordan (b <= 136), 3..4 register-tiled
-// (b <= 160), 5 global-memory Gauss-Jordan
-static int inv_class(int b) {
-    return b <= 32 ? 0 : b <= 64 ? 1 : b <= TCI_MAX ? 2 : b <= 144 ? 3 : b <= 160 ? 4 : 5;
-}
+// Rows of a level are inverted in groups of alike blocks: a launch takes the
+// cluster size and the panel warps of its largest one.
+static int inv_class(int b) { return b <= 64 ? 0 : b <= 136 ? 1 : b <= 208 ? 2 : b <= 320 ? 3 : b <= GJ_MAX ? 4 : 5; }
 
 // Levels, LD slots, GEMM tasks, device upload.
 static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluProgram& P) {
@@ -1390,8 +1386,7 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
         P.max_b = std::max(P.max_b, P.prow_b[pr]);
     }
     // factorisation schedule per forward level.  Rows of a level are ordered
-    // by block-size class so that each inverse launch uses the register tile
-    // that fits; products of blocks that the FP32 tensor-core kernels take
+    // by block-size class (inv_class); products of blocks that the FP32 tensor-core kernels take
     // come first in each level.
     std::vector<GemmTask> ltasks, stasks;
     std::vector<GemmPair> lpairs, spairs;
@@ -1407,9 +1402,10 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
                          [&](int32_t a, int32_t b2) { return inv_class(P.prow_b[a]) < inv_class(P.prow_b[b2]); });
         for (int i = P.fwd_ptr[l]; i < P.fwd_ptr[l + 1];) {
             const int cls = inv_class(P.prow_b[P.fwd_rows[i]]);
-            int j = i;
-            while (j < P.fwd_ptr[l + 1] && inv_class(P.prow_b[P.fwd_rows[j]]) == cls) ++j;
-            P.inv_seg.push_back({i, j - i, cls});
+            int j = i, bmax = 0;
+            for (; j < P.fwd_ptr[l + 1] && inv_class(P.prow_b[P.fwd_rows[j]]) == cls; ++j)
+                bmax = std::max(bmax, P.prow_b[P.fwd_rows[j]]);
+            P.inv_seg.push_back({i, j - i, bmax});
             i = j;
         }
         P.inv_seg_ptr[l + 1] = (int)P.inv_seg.size();
@@ -1567,282 +1563,57 @@ extern "C" int chidg_gpu_precon_stamp(chidg_gpu_precon* M, int64_t* s) {
     return CHIDG_GPU_OK;
 }
 
-namespace chidg {
-// Blocks of 161..352 rows (P3 with five fields: 320): Gauss-Jordan with
-// partial pivoting, one row of the block per thread.  The pivot search, the
-// scaling and the elimination of a panel's columns then run in registers,
-// with one barrier a step (each warp posts its best candidate row and key in
-// a buffer of the step's parity; every warp then picks the winner), and
-// rows are never interchanged: as in the 136-row tensor-core kernel, the
-// pivot of column k is the entry of largest magnitude among the rows not yet
-// used as pivots (the first such row on ties), step k records its row p_k,
-// and the permutation is undone at the end.  Panels of RP_NB columns: after a
-// panel's steps, every other column c becomes c with rows {p_k} zeroed plus
-// P X_c, P the eliminated panel and X_c the old values of c in rows p_k (a
-// rank-RP_NB update on the FP64 tensor cores, m16n8k8 tiles).  The stored
-// matrix S then satisfies S(p_k, j) = inv(A)(k, p_j): the write-back permutes
-// each column's rows (a warp a column, through registers) and then the
-// columns along the cycles of the pivot order (a thread a row).  Dynamic
-// shared memory: 2 RP_NB max_b doubles (the panel and the pivot rows' values).
-constexpr int RP_NB = 32, RP_THREADS = 512, RP_MAX = 352;
-static __global__ void __launch_bounds__(RP_THREADS, 1)
-    k_block_inverse_rows(double* __restrict__ LD, const int64_t* __restrict__ dinv_off, const int32_t* __restrict__ prow_b,
-                         const int32_t* __restrict__ prow_elem, const int32_t* __restrict__ rows, int row_begin,
-                         int* __restrict__ status, int max_b) {
-    extern __shared__ double rp_smem[];
-    constexpr int NW = RP_THREADS / 32;
-    // per step (double-buffered by step parity): each warp's best candidate,
-    // its key and its row values
-    __shared__ __align__(16) double cand_row[2][NW][RP_NB];
-    __shared__ unsigned ck_hi[2][NW], ck_lo[2][NW];
-    __shared__ int ck_row[2][NW];
-    __shared__ int piv[RP_MAX], stepof[RP_MAX];
-    __shared__ unsigned char visited[RP_MAX];
-    const int prow = rows[row_begin + blockIdx.x];
-    const int b = prow_b[prow];
-    double* D = LD + dinv_off[prow];
-    double* Pn = rp_smem;                         // [RP_NB][max_b]: eliminated panel, column t at Pn[t * max_b]
-    double* X = Pn + (size_t)RP_NB * max_b;       // [RP_NB][max_b]: X[t * max_b + j] = old D(p_t, j)
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int i = tid;                            // this thread's row
-    const bool mine = i < b;
-    bool used = false, singular = false;
-    for (int q = tid; q < RP_MAX; q += RP_THREADS) { stepof[q] = -1; visited[q] = 0; }
-    __syncthreads();
-    for (int k0 = 0; k0 < b; k0 += RP_NB) {
-        const int nb = min(RP_NB, b - k0);
-        double r[RP_NB];
-#pragma unroll
-        for (int c = 0; c < RP_NB; ++c) r[c] = (mine && c < nb) ? D[i + (int64_t)(k0 + c) * b] : 0.0;
-#pragma unroll
-        for (int t = 0; t < RP_NB; ++t) {
-            if (t >= nb) break;
-            const int k = k0 + t;
-            // pivot: the largest |r[t]| among unused rows (integer keys: the
-            // bits of |v| are monotone in |v|, a NaN sorts above +inf; key + 1
-            // marks a candidate), first row on ties
-            const unsigned long long kb = (unsigned long long)__double_as_longlong(fabs(r[t]));
-            const unsigned long long key = (mine && !used) ? kb + 1ull : 0ull;
-            const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-            const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-            const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-            const unsigned cand = (hi == mhi && lo == mlo) ? (unsigned)i : 0xffffffffu;
-            const unsigned mrow = __reduce_min_sync(0xffffffffu, cand);
-            // the warp's candidate row and key, in this step's buffer; one
-            // barrier, then every warp picks the winner among the 16
-            const int buf = k & 1;
-            if ((unsigned)i == mrow) {
-#pragma unroll
-                for (int c = 0; c < RP_NB; c += 2)
-                    reinterpret_cast<double2*>(cand_row[buf][w])[c >> 1] = make_double2(r[c], r[c + 1]);
-            }
-            if (lane == 0) { ck_hi[buf][w] = mhi; ck_lo[buf][w] = mlo; ck_row[buf][w] = (int)mrow; }
-            __syncthreads();
-            const unsigned qh = lane < NW ? ck_hi[buf][lane] : 0u, ql = lane < NW ? ck_lo[buf][lane] : 0u;
-            const unsigned qr = lane < NW ? (unsigned)ck_row[buf][lane] : 0xffffffffu;
-            const unsigned gh = __reduce_max_sync(0xffffffffu, qh);
-            const unsigned gl = __reduce_max_sync(0xffffffffu, qh == gh ? ql : 0u);
-            // b - k >= 1 unused rows: some key is nonzero and p is a row
-            const int p = (int)__reduce_min_sync(0xffffffffu, (qh == gh && ql == gl) ? qr : 0xffffffffu);
-            const double* prow_s = cand_row[buf][p >> 5];
-            if (i == p) {
-                used = true;
-                piv[k] = p;
-                stepof[p] = k;
-            }
-            double pv = prow_s[t];
-            if (pv == 0.0) { singular = true; pv = 1.0; }
-            const double rcp = 1.0 / pv;
-            if (i == p) {
-#pragma unroll
-                for (int c = 0; c < RP_NB; ++c) r[c] = (c == t) ? rcp : r[c] * rcp;
-            } else {
-                const double f = r[t];
-#pragma unroll
-                for (int c = 0; c < RP_NB; c += 2) {
-                    const double2 pr2 = reinterpret_cast<const double2*>(prow_s)[c >> 1];
-                    r[c] = (c == t) ? -f * rcp : r[c] - f * (pr2.x * rcp);
-                    r[c + 1] = (c + 1 == t) ? -f * rcp : r[c + 1] - f * (pr2.y * rcp);
-                }
-            }
-        }
-        // the eliminated panel: back to its columns, and into shared memory;
-        // the old values of the panel's pivot rows in every other column
-        if (mine) {
-#pragma unroll
-            for (int c = 0; c < RP_NB; ++c)
-                if (c < nb) {
-                    D[i + (int64_t)(k0 + c) * b] = r[c];
-                    Pn[c * max_b + i] = r[c];
-                }
-        }
-        const int nout = b - nb;
-        for (int idx = tid; idx < nb * nout; idx += RP_THREADS) {
-            const int t = idx / nout, jj = idx - t * nout;
-            const int j = jj < k0 ? jj : jj + nb;
-            X[t * max_b + jj] = D[piv[k0 + t] + (int64_t)j * b];
-        }
-        __syncthreads();
-        // c <- c with rows {p_t} zeroed + P X_c for every column c outside the
-        // panel, on the FP64 tensor cores: a warp takes 16 x 16 output tiles
-        // (rows 16 tr.., outside-panel columns 16 tc..), two mma.sync m16n8k8
-        // per slice of 8 steps sharing the A fragment, P and X read from
-        // shared memory (entries past b rows, nb steps or the outside columns
-        // read as 0)
-        {
-            const int g = lane >> 2, tq = lane & 3;
-            const int ntr = (b + 15) / 16, ntc = (nout + 15) / 16;
-            for (int tile = w; tile < ntr * ntc; tile += NW) {
-                const int r0 = 16 * (tile % ntr), jj0 = 16 * (tile / ntr);
-                double d[2][4];
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int row = r0 + g + 8 * (e >> 1), jj = jj0 + 8 * h + 2 * tq + (e & 1);
-                        double base = 0.0;
-                        if (row < b && jj < nout) {
-                            const int st = stepof[row];
-                            base = (st >= k0 && st < k0 + nb) ? 0.0 : D[row + (int64_t)(jj < k0 ? jj : jj + nb) * b];
-                        }
-                        d[h][e] = base;
-                    }
-#pragma unroll
-                for (int k8 = 0; k8 < RP_NB; k8 += 8) {
-                    if (k8 >= nb) break;
-                    const int ka = k8 + tq, kb2 = k8 + tq + 4;
-                    const int ra = r0 + g, rb = r0 + g + 8;
-                    const double a0 = (ka < nb && ra < b) ? Pn[ka * max_b + ra] : 0.0;
-                    const double a1 = (ka < nb && rb < b) ? Pn[ka * max_b + rb] : 0.0;
-                    const double a2 = (kb2 < nb && ra < b) ? Pn[kb2 * max_b + ra] : 0.0;
-                    const double a3 = (kb2 < nb && rb < b) ? Pn[kb2 * max_b + rb] : 0.0;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int cj = jj0 + 8 * h + g;
-                        const double b0 = (ka < nb && cj < nout) ? X[ka * max_b + cj] : 0.0;
-                        const double b1 = (kb2 < nb && cj < nout) ? X[kb2 * max_b + cj] : 0.0;
-                        dmma_16x8x8(d[h][0], d[h][1], d[h][2], d[h][3], a0, a1, a2, a3, b0, b1);
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int row = r0 + g + 8 * (e >> 1), jj = jj0 + 8 * h + 2 * tq + (e & 1);
-                        if (row < b && jj < nout) D[row + (int64_t)(jj < k0 ? jj : jj + nb) * b] = d[h][e];
-                    }
-            }
-        }
-        __syncthreads();
-    }
-    // the cycles of the pivot order, marked once: visited[j] = 2 where a
-    // cycle of length > 1 starts (its smallest column), 1 elsewhere
-    if (tid == 0)
-        for (int j0 = 0; j0 < b; ++j0) {
-            if (visited[j0]) continue;
-            int cur = j0, n = 0;                          // piv is a permutation: at most b hops
-            do { visited[cur] = 1; cur = piv[cur]; } while (cur != j0 && ++n < b);
-            if (piv[j0] != j0) visited[j0] = 2;
-        }
-    // rows: S(i, j) -> (stepof[i], j), a warp per column through registers
-    constexpr int RPL = (RP_MAX + 31) / 32;
-    for (int j = w; j < b; j += RP_THREADS / 32) {
-        double* col = D + (int64_t)j * b;
-        double v[RPL];
-#pragma unroll
-        for (int q = 0; q < RPL; ++q) {
-            const int row = lane + 32 * q;
-            v[q] = row < b ? col[row] : 0.0;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < RPL; ++q) {
-            const int row = lane + 32 * q;
-            if (row < b) col[stepof[row]] = v[q];
-        }
-    }
-    __syncthreads();
-    // columns: column j -> column piv[j], along the cycles of piv; thread i
-    // carries row i (every thread follows the same cycles)
-    for (int j0 = 0; j0 < b; ++j0) {
-        if (visited[j0] != 2) continue;
-        double carry = mine ? D[i + (int64_t)j0 * b] : 0.0;
-        int cur = j0, n = 0;
-        do {
-            const int dst = piv[cur];
-            if (mine) {
-                const double tmp = D[i + (int64_t)dst * b];
-                D[i + (int64_t)dst * b] = carry;
-                carry = tmp;
-            }
-            cur = dst;
-        } while (cur != j0 && ++n < b);
-    }
-    if (singular && tid == 0) atomicMin(status, prow_elem[prow]);
-}
-}  // namespace chidg
-
-// CHIDG_INVERSE_PANELS=1: blocks of 161..352 rows on the shared-memory panel
-// kernel instead of the row-per-thread kernel (comparison runs)
-static bool inverse_panels_env() {
-    static const bool v = [] {
-        const char* e = std::getenv("CHIDG_INVERSE_PANELS");
-        return e && e[0] == '1';
-    }();
-    return v;
-}
-
-static int launch_inverse(chidg_gpu_precon* M, int row_begin, int count, int cls) {
+// the inverses of rows row_begin .. + count of the factorisation order, blocks of at most bmax rows
+static int launch_inverse(chidg_gpu_precon* M, int row_begin, int count, int bmax) {
     chidg_gpu_ctx* ctx = M->ctx;
     IluProgram& P = M->P;
     double* LD = (double*)M->LD.ptr;
-#define CHIDG_INV2(CL, RW)                                                                                       \
-    k_block_inverse3<CL, RW><<<count, 512, 0, ctx->stream>>>(LD, (const int64_t*)P.d_dinv_off.ptr,                  \
-                                                             (const int32_t*)P.d_prow_b.ptr,                        \
-                                                             (const int32_t*)P.d_prow_elem.ptr,                     \
-                                                             (const int32_t*)P.d_fwd_rows.ptr, row_begin, ctx->d_status)
-    switch (cls) {
-        case 0: CHIDG_INV2(1, 2); break;
-        case 1: CHIDG_INV2(2, 4); break;
-        case 2:
-            k_block_inverse_tc<<<count, TCI_THREADS, 0, ctx->stream>>>(LD, (const int64_t*)P.d_dinv_off.ptr,
-                                                                     (const int32_t*)P.d_prow_b.ptr,
-                                                                     (const int32_t*)P.d_prow_elem.ptr,
-                                                                     (const int32_t*)P.d_fwd_rows.ptr, row_begin, ctx->d_status);
-            break;
-        case 3: CHIDG_INV2(5, 9); break;
-        case 4: CHIDG_INV2(5, 10); break;
-        default: {
-            // 161..1024 rows: panels of 32 columns (16 above 352 rows, 8 above
-            // 704), (2 NB + 1) b doubles of shared memory
-            int st = ensure(ctx, M->piv_scratch, sizeof(int) * 1024 * (size_t)std::max(count, 1));
-            if (st) return st;
-            const int bmax = P.max_b;
-            auto go = [&](auto kern, int nbw) -> int {
-                const size_t smem = sizeof(double) * (size_t)(2 * nbw + 1) * bmax;
-                int s2 = raise_smem_limit((const void*)kern, smem);
-                if (s2) return fail(ctx, s2, "panel inverse shared memory");
-                kern<<<count, 256, smem, ctx->stream>>>(LD, (const int64_t*)P.d_dinv_off.ptr, (const int32_t*)P.d_prow_b.ptr,
-                                                        (const int32_t*)P.d_prow_elem.ptr, (const int32_t*)P.d_fwd_rows.ptr,
-                                                        row_begin, ctx->d_status, (int*)M->piv_scratch.ptr);
-                return CHIDG_GPU_OK;
-            };
-            if (bmax <= RP_MAX && !inverse_panels_env()) {
-                // a row per thread, panels in registers (k_block_inverse_rows)
-                const size_t smem = sizeof(double) * 2 * RP_NB * (size_t)bmax;
-                if ((st = raise_smem_limit((const void*)k_block_inverse_rows, smem)))
-                    return fail(ctx, st, "row inverse shared memory");
-                k_block_inverse_rows<<<count, RP_THREADS, smem, ctx->stream>>>(
-                    LD, (const int64_t*)P.d_dinv_off.ptr, (const int32_t*)P.d_prow_b.ptr, (const int32_t*)P.d_prow_elem.ptr,
-                    (const int32_t*)P.d_fwd_rows.ptr, row_begin, ctx->d_status, bmax);
-            } else if (bmax <= 352) st = go(k_block_inverse_panels<32>, 32);
-            else if (bmax <= 704) st = go(k_block_inverse_panels<16>, 16);
-            else st = go(k_block_inverse_panels<8>, 8);
-            if (st) return st;
-        }
+    const int64_t* off = (const int64_t*)P.d_dinv_off.ptr;
+    const int32_t *pb = (const int32_t*)P.d_prow_b.ptr, *pe = (const int32_t*)P.d_prow_elem.ptr,
+                  *rows = (const int32_t*)P.d_fwd_rows.ptr;
+    int st;
+    if (bmax <= GJ_MAX) {
+        const int C = gj_cluster(bmax), T = (gj_rows(bmax) + 31) / 32;
+        // update warps (and, in a cluster, the one that pushes the panels): the
+        // products take about as long as the panel with two tiles a warp
+        const int threads = 32 * std::min(GJ_THREADS / 32, T + (bmax <= 64 ? 2 : 7));
+        const size_t smem = gj_smem(bmax, C);
+        auto go = [&](auto kern) -> int {
+            const int s2 = raise_smem_limit((const void*)kern, smem);
+            if (s2) return fail(ctx, s2, "block inverse shared memory");
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(count * C));
+            cfg.blockDim = dim3((unsigned)threads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = ctx->stream;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = (unsigned)C;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = C > 1 ? 1 : 0;
+            const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, LD, off, pb, pe, rows, row_begin, ctx->d_status, C, T);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                return cuda_fail(ctx, e, "k_block_inverse_gj");
+            }
+            return check_launch(ctx, "k_block_inverse_gj");
+        };
+        if (C == 1) return T <= 4 ? go(k_block_inverse_gj<false, 4>) : go(k_block_inverse_gj<false, 8>);
+        return T <= 8 ? go(k_block_inverse_gj<true, 8>) : go(k_block_inverse_gj<true, 12>);
     }
-#undef CHIDG_INV2
-    return check_launch(ctx, "k_block_inverse");
+    // larger blocks: panels of 16 columns (8 above 704 rows) in shared memory,
+    // (2 NB + 1) b doubles
+    if ((st = ensure(ctx, M->piv_scratch, sizeof(int) * 1024 * (size_t)std::max(count, 1)))) return st;
+    auto go = [&](auto kern, int nbw) -> int {
+        const size_t smem = sizeof(double) * (size_t)(2 * nbw + 1) * bmax;
+        const int s2 = raise_smem_limit((const void*)kern, smem);
+        if (s2) return fail(ctx, s2, "panel inverse shared memory");
+        kern<<<count, 256, smem, ctx->stream>>>(LD, off, pb, pe, rows, row_begin, ctx->d_status, (int*)M->piv_scratch.ptr);
+        return CHIDG_GPU_OK;
+    };
+    if ((st = bmax <= 704 ? go(k_block_inverse_panels<16>, 16) : go(k_block_inverse_panels<8>, 8))) return st;
+    return check_launch(ctx, "k_block_inverse_panels");
 }
 
 // precon%update for the mixed-precision inner solves (MIXED_FP32, MIXED_BF16):

@@ -4,7 +4,7 @@
 #include "kernels.cuh"
 #include "factor_gemm.cuh"
 #include "stream_sweep.cuh"
-#include "inverse_tc.cuh"
+#include "inverse_gj.cuh"
 #include "stream_matvec.cuh"
 #include "umma_gemm.cuh"
 
@@ -64,7 +64,7 @@ struct IluProgram {
     std::vector<int> fwd_ptr, bwd_ptr;
     std::vector<int> ltask_ptr, stask_ptr;      // factor products per level
     std::vector<int> ltask_small, stask_small;  // of them, those the FP32 kernels for small blocks take (first in the level)
-    std::vector<std::array<int, 3>> inv_seg;   // per level: (row_begin, count, register-tile class)
+    std::vector<std::array<int, 3>> inv_seg;   // per level: (row_begin, count, largest block)
     // task-split sweeps: tasks in hand-out order, partial offsets per entry
     int ntask_f = 0, ntask_b = 0;
     int64_t part_f = 0, part_b = 0;            // scratch sizes (values)

@@ -796,463 +796,11 @@ static __global__ void k_convert_dinv(const double* __restrict__ LD, float* __re
     for (int i = threadIdx.x; i < n; i += blockDim.x) LD32[o + i] = (float)LD[o + i];
 }
 
-// In-place inverse of one diagonal block per CTA: Gauss-Jordan with partial
-// (row) pivoting, restated from the textbook algorithm.  The pivot of column
-// k is the entry of largest magnitude among rows not yet used as pivots
-// (first such row on ties), which is the pivot DGETRF selects.  Rows are not
-// swapped physically: each thread keeps a fixed RPL x CPW register tile
-// (rows lane + 32*ri, columns warp + NW*cj) and the permutation is undone
-// when the result is written.  A zero pivot records the element in *status
-// (ESINGULAR) and leaves garbage, never traps.
-template <int RPL, int CPW, int NW>
-__global__ void __launch_bounds__(NW * 32) k_block_inverse(double* __restrict__ LD, const int64_t* __restrict__ dinv_off,
-                                                           const int32_t* __restrict__ prow_b,
-                                                           const int32_t* __restrict__ prow_elem,
-                                                           const int32_t* __restrict__ rows, int row_begin,
-                                                           int* __restrict__ status) {
-    constexpr int RMAX = 32 * RPL, CMAX = NW * CPW;
-    __shared__ double colbuf[2][RMAX];
-    __shared__ double rowbuf[2][CMAX];
-    __shared__ int used[RMAX];
-    __shared__ int pivrow[CMAX > RMAX ? CMAX : RMAX];
-    __shared__ int qinv[RMAX];
-    __shared__ int s_p;
-    __shared__ double s_piv;
-    const int prow = rows[row_begin + blockIdx.x];
-    const int b = prow_b[prow];
-    double* D = LD + dinv_off[prow];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double a[RPL][CPW];
-    #pragma unroll
-    for (int ri = 0; ri < RPL; ++ri)
-        #pragma unroll
-        for (int cj = 0; cj < CPW; ++cj) {
-            const int i = lane + 32 * ri, j = w + NW * cj;
-            a[ri][cj] = (i < b && j < b) ? D[i + (int64_t)j * b] : 0.0;
-        }
-    for (int i = threadIdx.x; i < RMAX; i += blockDim.x) used[i] = 0;
-    bool singular = false;
-    __syncthreads();
-    for (int k = 0; k < b; ++k) {
-        const int wk = k % NW, ck = k / NW, buf = k & 1;
-        if (w == wk) {
-            double best = -1.0;
-            int bi = 0x7fffffff;
-            #pragma unroll
-            for (int ri = 0; ri < RPL; ++ri) {
-                const int i = lane + 32 * ri;
-                double v = -1.0;
-                #pragma unroll
-                for (int cj = 0; cj < CPW; ++cj) if (cj == ck) v = fabs(a[ri][cj]);
-                if (!(v == v)) v = INFINITY;   // a NaN entry is taken as pivot so the NaN propagates
-                if (i < b && !used[i] && (v > best || (v == best && i < bi))) { best = v; bi = i; }
-            }
-            #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-            }
-            if (lane == (bi & 31)) {
-                const int rp = bi >> 5;
-                double pv = 0.0;
-                #pragma unroll
-                for (int ri = 0; ri < RPL; ++ri)
-                    #pragma unroll
-                    for (int cj = 0; cj < CPW; ++cj) if (ri == rp && cj == ck) pv = a[ri][cj];
-                s_p = bi;
-                s_piv = pv;
-                used[bi] = 1;
-                pivrow[k] = bi;
-            }
-        }
-        __syncthreads();
-        const int p = s_p;
-        double piv = s_piv;
-        if (piv == 0.0) { singular = true; piv = 1.0; }
-        const double rp = 1.0 / piv;
-        if (lane == (p & 31)) {
-            const int rip = p >> 5;
-            #pragma unroll
-            for (int cj = 0; cj < CPW; ++cj) {
-                const int j = w + NW * cj;
-                double v = 0.0;
-                #pragma unroll
-                for (int ri = 0; ri < RPL; ++ri) if (ri == rip) v = a[ri][cj];
-                if (j == k) v = 1.0;
-                if (j < CMAX) rowbuf[buf][j] = v * rp;
-            }
-        }
-        if (w == wk) {
-            #pragma unroll
-            for (int ri = 0; ri < RPL; ++ri) {
-                const int i = lane + 32 * ri;
-                double v = 0.0;
-                #pragma unroll
-                for (int cj = 0; cj < CPW; ++cj) if (cj == ck) v = a[ri][cj];
-                colbuf[buf][i] = (i == p) ? 0.0 : v;
-            }
-        }
-        __syncthreads();
-        #pragma unroll
-        for (int ri = 0; ri < RPL; ++ri) {
-            const int i = lane + 32 * ri;
-            const double f = colbuf[buf][i];
-            #pragma unroll
-            for (int cj = 0; cj < CPW; ++cj) {
-                const int j = w + NW * cj;
-                const double rv = rowbuf[buf][j];
-                if (i == p) a[ri][cj] = rv;
-                else {
-                    const double base = (j == k) ? 0.0 : a[ri][cj];
-                    a[ri][cj] = fma(-f, rv, base);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < b; k += blockDim.x) qinv[pivrow[k]] = k;
-    __syncthreads();
-    #pragma unroll
-    for (int ri = 0; ri < RPL; ++ri)
-        #pragma unroll
-        for (int cj = 0; cj < CPW; ++cj) {
-            const int i = lane + 32 * ri, j = w + NW * cj;
-            if (i < b && j < b) D[qinv[i] + (int64_t)pivrow[j] * b] = a[ri][cj];
-        }
-    if (singular && threadIdx.x == 0) atomicMin(status, prow_elem[prow]);
-}
-
-// In-place inverse, second layout: 16 warps, warp w owns rows w + 16*ri
-// (ri < RW), lane l owns columns l + 32*cl (cl < CL), so b <= min(32*CL, 16*RW).  The
-// pivot loop is split into a compile-time column slot ck and a runtime lane
-// lk (k = 32*ck + lk): every access to the pivot column is then a static
-// register index, and only the pivot row needs a runtime row select (done
-// by its owning warp alone).  Same pivoting rule and result as
-// k_block_inverse: Gauss-Jordan with implicit row pivoting, largest |a|
-// among unused rows (first on ties), permutation undone on the store.
-template <int CL, int RW>
-__global__ void __launch_bounds__(512) k_block_inverse2(double* __restrict__ LD, const int64_t* __restrict__ dinv_off,
-                                                       const int32_t* __restrict__ prow_b,
-                                                       const int32_t* __restrict__ prow_elem,
-                                                       const int32_t* __restrict__ rows, int row_begin,
-                                                       int* __restrict__ status) {
-    constexpr int NW = 16, NMAX = (32 * CL > NW * RW) ? 32 * CL : NW * RW;
-    __shared__ double colbuf[NMAX];
-    __shared__ double rowbuf[2][NMAX];
-    __shared__ double cand_v[NW];
-    __shared__ double cand_a[NW];
-    __shared__ int cand_i[NW];
-    __shared__ int pivrow[NMAX];
-    __shared__ int qinv[NMAX];
-    const int prow = rows[row_begin + blockIdx.x];
-    const int b = prow_b[prow];
-    double* D = LD + dinv_off[prow];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double a[RW][CL];
-    #pragma unroll
-    for (int ri = 0; ri < RW; ++ri)
-        #pragma unroll
-        for (int cl = 0; cl < CL; ++cl) {
-            const int i = w + NW * ri, j = lane + 32 * cl;
-            a[ri][cl] = (i < b && j < b) ? D[i + (int64_t)j * b] : 0.0;
-        }
-    unsigned used = 0;          // bit ri set: row w + NW*ri already used as a pivot
-    bool singular = false;
-    #pragma unroll
-    for (int ck = 0; ck < CL; ++ck) {
-        for (int lk = 0; lk < 32; ++lk) {
-            const int k = 32 * ck + lk;
-            if (k >= b) break;
-            const int buf = k & 1;
-            // (a) candidates of this warp's rows in column k; column k to colbuf
-            if (lane == lk) {
-                double best = -1.0, bestv = 0.0;
-                int bi = 0x7fffffff;
-                #pragma unroll
-                for (int ri = 0; ri < RW; ++ri) {
-                    const int i = w + NW * ri;
-                    if (i < b) {
-                        colbuf[i] = a[ri][ck];
-                        double m = fabs(a[ri][ck]);
-                        if (!(m == m)) m = INFINITY;   // a NaN pivot propagates
-                        if (!((used >> ri) & 1u) && (m > best || (m == best && i < bi))) { best = m; bi = i; bestv = a[ri][ck]; }
-                    }
-                }
-                cand_v[w] = best;
-                cand_a[w] = bestv;
-                cand_i[w] = bi;
-            }
-            __syncthreads();
-            // (b) every thread picks the pivot from the 16 candidates
-            double best = -1.0, piv = 0.0;
-            int p = 0x7fffffff;
-            #pragma unroll
-            for (int q = 0; q < NW; ++q) {
-                const double v = cand_v[q];
-                const int iq = cand_i[q];
-                if (v > best || (v == best && iq < p)) { best = v; p = iq; piv = cand_a[q]; }
-            }
-            if (piv == 0.0) { singular = true; piv = 1.0; }
-            const double rp = 1.0 / piv;
-            const int pw = p % NW, prr = p / NW;
-            if (w == pw) {
-                used |= 1u << prr;
-                #pragma unroll
-                for (int cl = 0; cl < CL; ++cl) {
-                    double v = 0.0;
-                    #pragma unroll
-                    for (int ri = 0; ri < RW; ++ri) if (ri == prr) v = a[ri][cl];
-                    if (cl == ck && lane == lk) v = 1.0;
-                    rowbuf[buf][lane + 32 * cl] = v * rp;
-                }
-            }
-            if (threadIdx.x == 0) pivrow[k] = p;
-            __syncthreads();
-            // (c) rank-1 update; row p becomes the scaled pivot row, column k
-            // becomes -a(i,k)/piv
-            double rv[CL];
-            #pragma unroll
-            for (int cl = 0; cl < CL; ++cl) rv[cl] = rowbuf[buf][lane + 32 * cl];
-            #pragma unroll
-            for (int ri = 0; ri < RW; ++ri) {
-                const int i = w + NW * ri;
-                if (i == p) {
-                    #pragma unroll
-                    for (int cl = 0; cl < CL; ++cl) a[ri][cl] = rv[cl];
-                } else {
-                    const double f = (i < b) ? colbuf[i] : 0.0;
-                    #pragma unroll
-                    for (int cl = 0; cl < CL; ++cl) a[ri][cl] = fma(-f, rv[cl], a[ri][cl]);
-                    if (lane == lk) a[ri][ck] = -f * rp;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < b; k += blockDim.x) qinv[pivrow[k]] = k;
-    __syncthreads();
-    #pragma unroll
-    for (int ri = 0; ri < RW; ++ri)
-        #pragma unroll
-        for (int cl = 0; cl < CL; ++cl) {
-            const int i = w + NW * ri, j = lane + 32 * cl;
-            if (i < b && j < b) D[qinv[i] + (int64_t)pivrow[j] * b] = a[ri][cl];
-        }
-    if (singular && threadIdx.x == 0) atomicMin(status, prow_elem[prow]);
-}
-
-// In-place inverse, third layout: the k_block_inverse2 tiles with one barrier
-// per pivot step.  Before the barrier every warp proposes the best unused row
-// of its own in column k, writes that candidate's value, reciprocal, index
-// and whole row (scaled later) into a double-buffered shared slot, and lane
-// lk writes the warp's part of column k.  After the barrier every warp picks
-// the winner with a 16-lane shuffle reduction (largest |a|, lowest row on
-// ties: the DGETRF choice) and reads the pivot row from the winner's slot, so
-// no warp has to wait for the owner of the pivot row.
-template <int CL, int RW>
-__global__ void __launch_bounds__(512) k_block_inverse3(double* __restrict__ LD, const int64_t* __restrict__ dinv_off,
-                                                       const int32_t* __restrict__ prow_b,
-                                                       const int32_t* __restrict__ prow_elem,
-                                                       const int32_t* __restrict__ rows, int row_begin,
-                                                       int* __restrict__ status) {
-    constexpr int NW = 16, NMAX = (32 * CL > NW * RW) ? 32 * CL : NW * RW;
-    __shared__ double colbuf[2][NMAX];
-    __shared__ double candrow[2][NW][32 * CL];
-    __shared__ double cand_v[2][NW];
-    __shared__ double cand_a[2][NW];
-    __shared__ int cand_i[2][NW];
-    __shared__ int pivrow[NMAX];
-    __shared__ int qinv[NMAX];
-    const int prow = rows[row_begin + blockIdx.x];
-    const int b = prow_b[prow];
-    double* D = LD + dinv_off[prow];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double a[RW][CL];
-    #pragma unroll
-    for (int ri = 0; ri < RW; ++ri)
-        #pragma unroll
-        for (int cl = 0; cl < CL; ++cl) {
-            const int i = w + NW * ri, j = lane + 32 * cl;
-            a[ri][cl] = (i < b && j < b) ? D[i + (int64_t)j * b] : 0.0;
-        }
-    unsigned used = 0;          // bit ri: row w + NW*ri already a pivot
-    bool singular = false;
-    #pragma unroll
-    for (int ck = 0; ck < CL; ++ck) {
-        for (int lk = 0; lk < 32; ++lk) {
-            const int k = 32 * ck + lk;
-            if (k >= b) break;
-            const int buf = k & 1;
-            // (a) this warp's candidate for column k
-            double best = -1.0, bestv = 0.0;
-            int bri = -1;
-            if (lane == lk) {
-                #pragma unroll
-                for (int ri = 0; ri < RW; ++ri) {
-                    const int i = w + NW * ri;
-                    if (i < b) {
-                        colbuf[buf][i] = a[ri][ck];
-                        double m = fabs(a[ri][ck]);
-                        if (!(m == m)) m = INFINITY;          // a NaN pivot propagates
-                        if (!((used >> ri) & 1u) && m > best) { best = m; bri = ri; bestv = a[ri][ck]; }
-                    }
-                }
-            }
-            best = __shfl_sync(0xffffffffu, best, lk);
-            bestv = __shfl_sync(0xffffffffu, bestv, lk);
-            bri = __shfl_sync(0xffffffffu, bri, lk);
-            if (bri >= 0) {
-                #pragma unroll
-                for (int cl = 0; cl < CL; ++cl) {
-                    double vsel = 0.0;
-                    #pragma unroll
-                    for (int ri = 0; ri < RW; ++ri) if (ri == bri) vsel = a[ri][cl];
-                    candrow[buf][w][lane + 32 * cl] = vsel;
-                }
-            }
-            if (lane == 0) {
-                cand_v[buf][w] = best;
-                cand_a[buf][w] = (bestv == 0.0) ? 1.0 : 1.0 / bestv;
-                cand_i[buf][w] = (bri >= 0) ? w + NW * bri : 0x7fffffff;
-            }
-            __syncthreads();
-            // (b) winner by shuffle reduction over the 16 candidates
-            double v = (lane < NW) ? cand_v[buf][lane] : -2.0;
-            int ii = (lane < NW) ? cand_i[buf][lane] : 0x7fffffff;
-            int src = lane;
-            #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) {
-                const double ov = __shfl_xor_sync(0xffffffffu, v, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, ii, o);
-                const int os = __shfl_xor_sync(0xffffffffu, src, o);
-                if (ov > v || (ov == v && oi < ii)) { v = ov; ii = oi; src = os; }
-            }
-            const int p = __shfl_sync(0xffffffffu, ii, 0);
-            const int ws = __shfl_sync(0xffffffffu, src, 0);
-            double rp = cand_a[buf][ws];
-            if (v == 0.0) singular = true;        // every candidate zero
-            if (w == (p % NW)) used |= 1u << (p / NW);
-            if (threadIdx.x == 0) pivrow[k] = p;
-            // (c) rank-1 update with the winner's row, scaled; row p becomes the
-            // scaled pivot row, column k becomes -a(i,k)/piv
-            double rv[CL];
-            #pragma unroll
-            for (int cl = 0; cl < CL; ++cl) {
-                const int j = lane + 32 * cl;
-                const double x = (cl == ck && lane == lk) ? 1.0 : candrow[buf][ws][j];
-                rv[cl] = x * rp;
-            }
-            #pragma unroll
-            for (int ri = 0; ri < RW; ++ri) {
-                const int i = w + NW * ri;
-                if (i == p) {
-                    #pragma unroll
-                    for (int cl = 0; cl < CL; ++cl) a[ri][cl] = rv[cl];
-                } else {
-                    const double f = (i < b) ? colbuf[buf][i] : 0.0;
-                    #pragma unroll
-                    for (int cl = 0; cl < CL; ++cl) a[ri][cl] = fma(-f, rv[cl], a[ri][cl]);
-                    if (lane == lk) a[ri][ck] = -f * rp;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < b; k += blockDim.x) qinv[pivrow[k]] = k;
-    __syncthreads();
-    #pragma unroll
-    for (int ri = 0; ri < RW; ++ri)
-        #pragma unroll
-        for (int cl = 0; cl < CL; ++cl) {
-            const int i = w + NW * ri, j = lane + 32 * cl;
-            if (i < b && j < b) D[qinv[i] + (int64_t)pivrow[j] * b] = a[ri][cl];
-        }
-    if (singular && threadIdx.x == 0) atomicMin(status, prow_elem[prow]);
-}
-
-// Same algorithm for blocks too large for the register tiles (b > 160):
-// one CTA, matrix kept in global memory (L2 resident), explicit row swaps.
-static __global__ void k_block_inverse_global(double* __restrict__ LD, const int64_t* __restrict__ dinv_off,
-                                       const int32_t* __restrict__ prow_b, const int32_t* __restrict__ prow_elem,
-                                       const int32_t* __restrict__ rows, int row_begin, int* __restrict__ status,
-                                       int* __restrict__ piv_scratch) {
-    __shared__ double sv[32];
-    __shared__ int si[32];
-    __shared__ int s_p;
-    __shared__ double colk[1024];
-    const int prow = rows[row_begin + blockIdx.x];
-    const int b = prow_b[prow];
-    double* D = LD + dinv_off[prow];
-    int* piv = piv_scratch + (int64_t)blockIdx.x * 1024;
-    bool singular = false;
-    for (int k = 0; k < b; ++k) {
-        double best = -1.0; int bi = 0x7fffffff;
-        for (int i = k + threadIdx.x; i < b; i += blockDim.x) {
-            double v = fabs(D[i + (int64_t)k * b]);
-            if (!(v == v)) v = INFINITY;
-            if (v > best || (v == best && i < bi)) { best = v; bi = i; }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bi; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double bb = -1.0; int ii = 0x7fffffff;
-            for (int q = 0; q < (int)(blockDim.x >> 5); ++q)
-                if (sv[q] > bb || (sv[q] == bb && si[q] < ii)) { bb = sv[q]; ii = si[q]; }
-            s_p = ii;
-            piv[k] = ii;
-        }
-        __syncthreads();
-        const int p = s_p;
-        if (p != k)
-            for (int j = threadIdx.x; j < b; j += blockDim.x) {
-                const double t = D[k + (int64_t)j * b];
-                D[k + (int64_t)j * b] = D[p + (int64_t)j * b];
-                D[p + (int64_t)j * b] = t;
-            }
-        __syncthreads();
-        double pv = D[k + (int64_t)k * b];
-        if (pv == 0.0) { singular = true; pv = 1.0; }
-        const double rp = 1.0 / pv;
-        __syncthreads();
-        for (int i = threadIdx.x; i < b; i += blockDim.x) colk[i] = (i == k) ? 0.0 : D[i + (int64_t)k * b];
-        __syncthreads();
-        for (int j = threadIdx.x; j < b; j += blockDim.x) {
-            const double v = (j == k) ? 1.0 : D[k + (int64_t)j * b];
-            D[k + (int64_t)j * b] = v * rp;
-        }
-        __syncthreads();
-        // row k is final for this step; every other row reads its multiplier
-        // from the saved column, so column k can be overwritten in place
-        for (int idx = threadIdx.x; idx < b * b; idx += blockDim.x) {
-            const int i = idx % b, j = idx / b;
-            if (i == k) continue;
-            const double base = (j == k) ? 0.0 : D[i + (int64_t)j * b];
-            D[i + (int64_t)j * b] = base - colk[i] * D[k + (int64_t)j * b];
-        }
-        __syncthreads();
-    }
-    // undo the row interchanges as column interchanges, last first
-    for (int k = b - 1; k >= 0; --k) {
-        const int p = piv[k];
-        if (p != k)
-            for (int i = threadIdx.x; i < b; i += blockDim.x) {
-                const double t = D[i + (int64_t)k * b];
-                D[i + (int64_t)k * b] = D[i + (int64_t)p * b];
-                D[i + (int64_t)p * b] = t;
-            }
-        __syncthreads();
-    }
-    if (singular && threadIdx.x == 0) atomicMin(status, prow_elem[prow]);
-}
-
-// Blocks of 161..1024 rows: the same Gauss-Jordan with row interchanges,
-// blocked by panels of NB columns.  A panel is factored in shared memory (its
+// In-place inverse of diagonal blocks of 385..1024 rows, one CTA a block:
+// Gauss-Jordan with partial (row) pivoting and row interchanges, blocked by
+// panels of NB columns.  The pivot of column k is the entry of largest
+// magnitude at or below the diagonal (the first such row on ties); a zero
+// pivot records the element in *status (ESINGULAR) and leaves garbage.  A panel is factored in shared memory (its
 // pivot searches, row interchanges, scaling and eliminations restricted to
 // the panel's columns; the interchanges are applied to the rest of the rows in
 // global memory at once).  Afterwards the panel holds G e_k for its pivot
@@ -1260,8 +808,7 @@ static __global__ void k_block_inverse_global(double* __restrict__ LD, const int
 // other column becomes D[:, j] + (G - I) D[k0:k0+nb, j]: a rank-nb update
 // computed from the panel and the pivot rows staged in shared memory, 8 x 4
 // outputs per thread.  Column interchanges undo the row interchanges at the
-// end, as in k_block_inverse_global.  Dynamic shared memory:
-// (2 NB + 1) b doubles.
+// end.  Dynamic shared memory: (2 NB + 1) b doubles.
 template <int NB>
 __global__ void __launch_bounds__(256) k_block_inverse_panels(double* __restrict__ LD, const int64_t* __restrict__ dinv_off,
                                                           const int32_t* __restrict__ prow_b,

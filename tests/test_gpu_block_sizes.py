@@ -1,0 +1,52 @@
+"""Factorisation and sweeps at the block sizes where their kernels change
+shape: the factor products' tiles (8 x 8 accumulators, CTA tiles of at most 80
+x 80), the inverses' panels of eight, row pairs of sixteen and cluster sizes
+(one CTA up to 136 rows, more above, another kernel above 384), the sweeps'
+one-task rows (up to 64) and column slices (three up to 160, eight above)."""
+import numpy as np
+import pytest
+
+from chidg_b200 import api, mesh
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# (fields, modes): block size is their product
+SIZES = [(1, 1), (7, 1), (1, 8), (3, 3), (5, 8), (13, 5), (8, 10), (27, 3), (1, 127), (17, 8), (1, 137), (32, 5), (7, 23),
+         (13, 16), (11, 19), (7, 40), (64, 5), (3, 107), (128, 3), (5, 77)]
+
+
+def _relerr(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("nvars,nterms", SIZES, ids=[f"b{v * t}" for v, t in SIZES])
+def test_factors_and_sweeps_by_block_size(nvars, nterms):
+    pat = mesh.box_pattern(2, 2, 2 if nvars * nterms < 200 else 1, nvars, nterms)
+    vals = mesh.synth_values(pat, seed=61)
+    # rows of the diagonal blocks in another order: pivots off the diagonal
+    rng = np.random.default_rng(62)
+    voff, _ = pat.value_offsets()
+    b = nvars * nterms
+    for k in np.nonzero(np.asarray(pat.blk_face) == mesh.DIAG)[0][::2]:
+        blk = vals[voff[k]:voff[k] + b * b].reshape(b, b)            # [column, row]
+        blk[:] = blk[:, rng.permutation(b)]
+    v = mesh.synth_vector(pat.vector_size(), seed=63)
+    Ao = O.OracleMatrix(pat)
+    Ao.set_values(vals)
+    Ag = api.ChidgMatrix(pat)
+    Ag.upload(vals)
+    Mo, Mg = O.OraclePrecon(Ao, "ilu0"), api.create_preconditioner("ilu0")
+    Mo.update()
+    Mg.update(Ag)
+    LDo, LDg = Mo.LD(), Mg.LD()
+    # the permuted systems are worse conditioned: a bound relative to the block
+    # inverses' condition, measured in FP64 by numpy
+    dk = np.nonzero(np.asarray(pat.blk_face) == mesh.DIAG)[0]
+    cond = max(np.linalg.cond(LDo[voff[k]:voff[k] + b * b].reshape(b, b)) for k in dk)
+    tol = 64 * b * np.finfo(float).eps * max(1.0, cond)
+    for k in range(pat.nblocks):
+        o = LDo[voff[k]:voff[k] + b * b]
+        if np.any(o):
+            assert _relerr(LDg[voff[k]:voff[k] + b * b], o) < tol
+    assert _relerr(Mg.apply(Ag, api.ChidgVector(Ag, v)).download(), Mo.apply(v)) < tol
