@@ -1390,6 +1390,7 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
     // come first in each level.
     std::vector<GemmTask> ltasks, stasks;
     std::vector<GemmPair> lpairs, spairs;
+    std::vector<int32_t> ltask_of;          // first L task of the row at each position of fwd_rows (small blocks)
     P.ltask_ptr.assign(P.fwd_ptr.size(), 0);
     P.stask_ptr.assign(P.fwd_ptr.size(), 0);
     P.ltask_small.assign(P.fwd_ptr.size(), 0);
@@ -1415,6 +1416,7 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
             for (int i = P.fwd_ptr[l]; i < P.fwd_ptr[l + 1]; ++i) {
                 const int pr = P.fwd_rows[i];
                 const int b = P.prow_b[pr];
+                if (pass == 0) ltask_of.push_back((int32_t)ltasks.size());
                 for (auto& en : P.lo[pr]) {
                     // L = A_lower * inv(D_parent)      (precon_ILU0.f90:231)
                     const bool small = b <= FACTOR32_SMALL && en.nc <= FACTOR32_SMALL;
@@ -1459,7 +1461,7 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
         (st = upload_array(ctx, P.d_up_nc, up_nc)) || (st = upload_array(ctx, P.d_fwd_rows, P.fwd_rows)) ||
         (st = upload_array(ctx, P.d_bwd_rows, P.bwd_rows)) || (st = upload_array(ctx, P.d_ltasks, ltasks)) ||
         (st = upload_array(ctx, P.d_lpairs, lpairs)) || (st = upload_array(ctx, P.d_stasks, stasks)) ||
-        (st = upload_array(ctx, P.d_spairs, spairs)))
+        (st = upload_array(ctx, P.d_spairs, spairs)) || (st = upload_array(ctx, P.d_ltask_of, ltask_of)))
         return st;
     P.rows.prow_b = (const int32_t*)P.d_prow_b.ptr;
     P.rows.v_off = (const int64_t*)P.d_v_off.ptr;
@@ -1486,7 +1488,7 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
 void chidg::release_program(IluProgram& P) {
     for (Buffer* b : {&P.d_prow_b, &P.d_prow_elem, &P.d_v_off, &P.d_z_off, &P.d_dinv_off, &P.d_lo_ptr, &P.d_lo_L,
                       &P.d_lo_par, &P.d_lo_nc, &P.d_up_ptr, &P.d_up_U, &P.d_up_par, &P.d_up_nc, &P.d_fwd_rows,
-                      &P.d_bwd_rows, &P.d_ltasks, &P.d_lpairs, &P.d_stasks, &P.d_spairs, &P.d_tf_row, &P.d_tf_ent,
+                      &P.d_bwd_rows, &P.d_ltasks, &P.d_lpairs, &P.d_stasks, &P.d_spairs, &P.d_ltask_of, &P.d_tf_row, &P.d_tf_ent,
                       &P.d_tb_row, &P.d_tb_ent, &P.d_poff_f, &P.d_poff_b, &P.d_sb_row, &P.d_sb_ent, &P.d_asm_ptr,
                       &P.d_asm_src, &P.d_asm_r0, &P.d_asm_c0, &P.d_asm_nr, &P.d_asm_nc, &P.d_bmv_row, &P.d_bmv_ent,
                       &P.d_col_prow, &P.d_mv_skip})
@@ -1786,7 +1788,26 @@ extern "C" int chidg_gpu_precon_update(chidg_gpu_precon* M, chidg_gpu_matrix* A,
                                                          (const int32_t*)P.d_asm_nr.ptr, (const int32_t*)P.d_asm_nc.ptr);
         if ((st = check_launch(ctx, "k_assemble_rows"))) return st;
     }
-    for (int l = 0; l < nlev; ++l) {
+    // one launch for programmes of small blocks, else three a wavefront
+    const bool by_rows = P.max_b <= FR_MAX && !P.assembled;
+    if (by_rows) {
+        const size_t smem = fr_smem(P.max_b);
+        if ((st = raise_smem_limit((const void*)k_factor_rows, smem))) return fail(ctx, st, "factor rows shared memory");
+        const int per_sm = resident_ctas((const void*)k_factor_rows, FG_THREADS, smem);
+        if (per_sm < 1) return fail(ctx, CHIDG_GPU_EINVAL, "factor rows: does not fit an SM");
+        unsigned* sync = (unsigned*)M->sync.ptr;
+        cudaMemsetAsync(sync, 0, sizeof(unsigned), ctx->stream);
+        cudaMemsetAsync(ctx->d_scal + kSlotStatus, 0, sizeof(double), ctx->stream);
+        const FactorRows FR{(const GemmTask*)P.d_ltasks.ptr, (const GemmTask*)P.d_stasks.ptr, (const GemmPair*)P.d_lpairs.ptr,
+                            (const GemmPair*)P.d_spairs.ptr, (const int32_t*)P.d_fwd_rows.ptr, P.rows.prow_b,
+                            (const int32_t*)P.d_prow_elem.ptr, P.rows.lo_ptr, P.rows.lo_par, (const int32_t*)P.d_ltask_of.ptr,
+                            P.rows.dinv_off, P.nprow};
+        SweepSync S{sync, sync + 2, ++M->epoch, (int*)(ctx->d_scal + kSlotStatus), kSpinLimit};
+        k_factor_rows<<<std::min(P.nprow, per_sm * ctx->nsm), FG_THREADS, smem, ctx->stream>>>(
+            FR, (const double*)A->val.ptr, (double*)M->LD.ptr, S, ctx->d_status);
+        if ((st = check_launch(ctx, "k_factor_rows"))) return st;
+    }
+    for (int l = 0; l < nlev && !by_rows; ++l) {
         const int pg = prof_begin(ctx, kProfFactorGemm);
         const int nl = P.ltask_ptr[l + 1] - P.ltask_ptr[l], ns = P.stask_ptr[l + 1] - P.stask_ptr[l];
         if (nl > 0) {
@@ -1809,6 +1830,11 @@ extern "C" int chidg_gpu_precon_update(chidg_gpu_precon* M, chidg_gpu_matrix* A,
     }
     prof_end(ctx, ph);
     cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    if (by_rows) {
+        double w = 0.0;
+        if ((st = fetch_scalars(ctx, kSlotStatus, 1, &w))) return st;
+        if ((st = status_word(ctx, w))) return st;
+    }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "precon update");
     if (ctx->h_status[0] != INT_MAX) {

@@ -5,9 +5,11 @@
 #include "factor_gemm.cuh"
 #include "stream_sweep.cuh"
 #include "inverse_gj.cuh"
+#include "factor_rows.cuh"
 #include "stream_matvec.cuh"
 #include "umma_gemm.cuh"
 
+#include <algorithm>
 #include <array>
 #include <cmath>
 #include <cstdint>
@@ -86,7 +88,7 @@ struct IluProgram {
     Buffer d_asm_ptr, d_asm_src, d_asm_r0, d_asm_c0, d_asm_nr, d_asm_nc;
     std::vector<int> inv_seg_ptr;
     Buffer d_prow_b, d_prow_elem, d_v_off, d_z_off, d_dinv_off, d_lo_ptr, d_lo_L, d_lo_par, d_lo_nc, d_up_ptr,
-        d_up_U, d_up_par, d_up_nc, d_fwd_rows, d_bwd_rows, d_ltasks, d_lpairs, d_stasks, d_spairs;
+        d_up_U, d_up_par, d_up_nc, d_fwd_rows, d_bwd_rows, d_ltasks, d_lpairs, d_stasks, d_spairs, d_ltask_of;
     IluRows rows{};
 };
 

@@ -161,16 +161,15 @@ __device__ __forceinline__ void fg_walk(const FgTile& T, const GemmPair* __restr
     }
 }
 
-static __global__ void __launch_bounds__(FG_THREADS, 3)
-    k_task_gemm_f64(const GemmTask* __restrict__ tasks, const GemmPair* __restrict__ pairs, int parts_m, int parts_n,
-                    const double* Abase, const double* Bbase, const double* Cinit, double* Cbase, double sgn) {
-    extern __shared__ __align__(16) double fg_smem[];
-    const int tiles = parts_m * parts_n;
+// CTA tile (im, in) of task t, by the FG_THREADS threads of a CTA; rot turns the
+// warps' quarters.  smem: FG_STAGES * FG_STAGE doubles.
+__device__ __forceinline__ void fg_tile(const GemmTask& t, int im, int in, int rot, const GemmPair* __restrict__ pairs,
+                                        const double* Abase, const double* Bbase, const double* Cinit, double* Cbase,
+                                        double sgn, double* fg_smem) {
     FgTile T;
-    T.t = tasks[blockIdx.x / tiles];
-    const int tile = blockIdx.x % tiles;
+    T.t = t;
     // the CTA's 8 x 8 tiles [ti0, ti0 + tm) x [tj0, tj0 + tn) of the output
-    const int pm = fg_parts(T.t.m), pn = fg_parts(T.t.n), im = tile % parts_m, in = tile / parts_m;
+    const int pm = fg_parts(T.t.m), pn = fg_parts(T.t.n);
     if (im >= pm || in >= pn) return;
     const int t8m = (T.t.m + 7) / 8, t8n = (T.t.n + 7) / 8;
     const int ti0 = t8m * im / pm, tj0 = t8n * in / pn;
@@ -181,7 +180,7 @@ static __global__ void __launch_bounds__(FG_THREADS, 3)
     T.n = min(8 * tn, T.t.n - T.c0);
     // the warp's quarter; the larger quarters of odd tile counts rotate over
     // the warps (the sub-cores) with the CTA
-    const int role = ((threadIdx.x >> 5) + blockIdx.x) & 3;
+    const int role = ((threadIdx.x >> 5) + rot) & 3;
     const int hm = (tm + 1) / 2, hn = (tn + 1) / 2;
     T.wi0 = (role & 1) ? hm : 0;
     T.wj0 = (role >> 1) ? hn : 0;
@@ -223,6 +222,15 @@ static __global__ void __launch_bounds__(FG_THREADS, 3)
                 if (j < T.n && i < T.m) C[i + (int64_t)j * T.t.m] = ci[u][r] + sgn * fg_smem[j * FG_LDA + i];
             }
     }
+}
+
+static __global__ void __launch_bounds__(FG_THREADS, 3)
+    k_task_gemm_f64(const GemmTask* __restrict__ tasks, const GemmPair* __restrict__ pairs, int parts_m, int parts_n,
+                    const double* Abase, const double* Bbase, const double* Cinit, double* Cbase, double sgn) {
+    extern __shared__ __align__(16) double fg_smem[];
+    const int tiles = parts_m * parts_n, tile = blockIdx.x % tiles;
+    fg_tile(tasks[blockIdx.x / tiles], tile % parts_m, tile / parts_m, blockIdx.x, pairs, Abase, Bbase, Cinit, Cbase, sgn,
+            fg_smem);
 }
 
 }  // namespace chidg

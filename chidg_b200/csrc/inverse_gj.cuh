@@ -171,18 +171,13 @@ __device__ __forceinline__ void gj_mma_rows(const double* S, int LD, const doubl
     a[3] = p[4 * LDP + 8];
 }
 
-// MAXT: at least T, a multiple of 4
+// one block D (b x b, column-major) in place, by the CTAs of a cluster of C
+// (CL) or one CTA; T of the CTA's warps are the panel warps (MAXT: at least T, a
+// multiple of 4).  raw: gj_smem(b, C) bytes.
 template <bool CL, int MAXT>
-static __global__ void __launch_bounds__(GJ_THREADS, 1)
-    k_block_inverse_gj(double* __restrict__ LD_, const int64_t* __restrict__ dinv_off, const int32_t* __restrict__ prow_b,
-                       const int32_t* __restrict__ prow_elem, const int32_t* __restrict__ rows, int row_begin,
-                       int* __restrict__ status, int C, int T) {
-    extern __shared__ __align__(128) unsigned char gj_raw[];
+__device__ __forceinline__ void gj_block(unsigned char* gj_raw, double* D, int b, int elem, int* status, int C, int T) {
     GjShared& sh = *reinterpret_cast<GjShared*>(gj_raw);
     const uint32_t rank = CL ? cluster_rank() : 0;
-    const int prow = rows[row_begin + (CL ? blockIdx.x / C : blockIdx.x)];
-    const int b = prow_b[prow];
-    double* D = LD_ + dinv_off[prow];
     const int nt8 = (b + 7) / 8, tc = (nt8 + C - 1) / C;          // tiles of the block, of a CTA
     const int first = min((int)rank * tc, nt8), ntl = min(tc, nt8 - first);
     const int rp = gj_rows(b), LD = rp + 2, LDP = rp + 4, PB = gj_panel(b);
@@ -464,7 +459,7 @@ static __global__ void __launch_bounds__(GJ_THREADS, 1)
         }
     }
     if (limit == 0) singular = true;
-    if (singular && lane == 0) atomicMin(status, prow_elem[prow]);
+    if (singular && lane == 0) atomicMin(status, elem);
     __syncthreads();
     if (CL) cluster_barrier();                    // no CTA leaves while another may write to its shared memory
     // inv(A)(k, p_j) = S(p_k, j); the lane's pivots are the same in every column
@@ -479,6 +474,16 @@ static __global__ void __launch_bounds__(GJ_THREADS, 1)
         for (int q = 0; q < GJ_MAXT; ++q)
             if (lane + 32 * q < b) out[32 * q] = S[c * LD + pk[q]];
     }
+}
+
+template <bool CL, int MAXT>
+static __global__ void __launch_bounds__(GJ_THREADS, 1)
+    k_block_inverse_gj(double* __restrict__ LD_, const int64_t* __restrict__ dinv_off, const int32_t* __restrict__ prow_b,
+                       const int32_t* __restrict__ prow_elem, const int32_t* __restrict__ rows, int row_begin,
+                       int* __restrict__ status, int C, int T) {
+    extern __shared__ __align__(128) unsigned char gj_raw[];
+    const int prow = rows[row_begin + (CL ? blockIdx.x / C : blockIdx.x)];
+    gj_block<CL, MAXT>(gj_raw, LD_ + dinv_off[prow], prow_b[prow], prow_elem[prow], status, C, T);
 }
 
 }  // namespace chidg
