@@ -390,7 +390,7 @@ template <typename T>
 struct BatchEngine {
     chidg_gpu_ctx* ctx = nullptr;
     chidg_gpu_matrix* A = nullptr;           // the operator: A, or A^T
-    chidg_gpu_precon* M = nullptr;           // set graph_safe while a sequence is captured
+    chidg_gpu_precon* M = nullptr;
     Segs g;
     BatchBuffers* BB = nullptr;              // state, partials, row sums, pinned counter and events
     Workspace* ws = nullptr;                 // Krylov basis and work vectors
@@ -564,16 +564,13 @@ int BatchEngine<T>::run(const T* bb, T* xx, std::vector<int64_t> key) {
         GR.step.clear();
     }
     GR.seen++;
-    // graphs need the streamed sweeps' flags reset inside each replay; the
-    // preconditioner records that it runs in captured sequences
+    // (the streamed sweeps clear their flags and counts inside each replay)
     const bool use = GR.seen >= 2 && !ctx->profiling && capturable && graphs_enabled();
     if (use && !GR.start) {
-        M->graph_safe = true;
         GR.start.reset(new GraphPiece());
         GR.end.reset(new GraphPiece());
         int st;
         if ((st = capture(ctx, *GR.start, seq_start)) || (st = capture(ctx, *GR.end, seq_end))) {
-            M->graph_safe = false;
             GR.start.reset();
             GR.end.reset();
             return st;
@@ -582,14 +579,12 @@ int BatchEngine<T>::run(const T* bb, T* xx, std::vector<int64_t> key) {
         for (int j = 1; j <= m; ++j) {
             GR.step[j - 1].reset(new GraphPiece());
             if ((st = capture(ctx, *GR.step[j - 1], [&]() { return seq_step(j); }))) {
-                M->graph_safe = false;
                 GR.start.reset();
                 GR.end.reset();
                 GR.step.clear();
                 return st;
             }
         }
-        M->graph_safe = false;
     }
     auto exec = [&](GraphPiece* gp, const std::function<int()>& eager) -> int {
         if (gp) {

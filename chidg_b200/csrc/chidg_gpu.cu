@@ -1267,6 +1267,191 @@ static int build_rasilu0(const chidg_gpu_matrix* A, IluProgram& P, std::string& 
 // cluster size and the panel warps of its largest one.
 static int inv_class(int b) { return b <= 64 ? 0 : b <= 136 ? 1 : b <= 208 ? 2 : b <= 320 ? 3 : b <= GJ_MAX ? 4 : 5; }
 
+// Which rows of a streamed sweep are one task, and where every row's partial
+// sums go.  Forward: a vector per slice of every entry; backward: the same (one
+// vector for a one-task row), then one per slice of inv(D).
+static void stream_layout(IluProgram& P) {
+    const int np = (int)P.prow_b.size();
+    P.part_s = 1;
+    P.max_row_task_cols = 0;
+    P.no_lower = true;
+    for (const auto& ents : P.lo) P.no_lower = P.no_lower && ents.empty();
+    for (int fwd = 1; fwd >= 0; --fwd) {
+        std::vector<uint8_t>& whole = fwd ? P.whole_f : P.whole_b;
+        std::vector<int64_t>& base = fwd ? P.base_f : P.base_u;
+        whole.assign(np, 0);
+        base.assign(np, 0);
+        if (!fwd) P.base_d.assign(np, 0);
+        int64_t size = 0;
+        for (int pr = 0; pr < np; ++pr) {
+            const auto& ents = (fwd ? P.lo : P.up)[pr];
+            const int b = P.prow_b[pr], ns = sweep_slices(b);
+            int cols = 0;
+            for (const auto& en : ents) cols += en.nc;
+            base[pr] = size;
+            if (b <= SW_ROW_B && cols <= SW_ROW_COLS) {
+                whole[pr] = 1;
+                P.max_row_task_cols = std::max(P.max_row_task_cols, std::max(cols, b));
+                if (!fwd && !ents.empty()) size += b;
+                continue;
+            }
+            size += (int64_t)b * ns * ents.size();
+            if (!fwd) {
+                P.base_d[pr] = size;
+                size += (int64_t)b * ns;
+            }
+        }
+        P.part_s = std::max(P.part_s, size);
+    }
+}
+
+// Tasks in key order (those of one key as added): added once to count them and
+// once more, after place(), to be stored.
+struct KeyedTasks {
+    int first;                        // the smallest key
+    std::vector<int64_t> at;          // tasks of a key; then where its next one goes
+    std::vector<StreamTask> task;
+    bool placing = false;
+    explicit KeyedTasks(int smallest) : first(smallest) {}
+    void add(int key, const StreamTask& t) {
+        const size_t k = (size_t)(key - first);
+        if (placing) {
+            task[(size_t)at[k]++] = t;
+            return;
+        }
+        if (at.size() <= k) at.resize(k + 1, 0);
+        ++at[k];
+    }
+    void place() {
+        int64_t n = 0;
+        for (int64_t& a : at) {
+            const int64_t here = a;
+            a = n;
+            n += here;
+        }
+        task.resize((size_t)n);
+        placing = true;
+    }
+};
+
+// The tasks of a streamed sweep with their keys: a slice of an entry follows
+// the level of the row it waits for (2 lev(parent)), a whole row and the slices
+// of inv(D) come just before the tasks that wait for the row (2 lev(row) - 1).  A
+// task waits only for rows all of whose tasks have smaller keys.  Keys are
+// scaled so that other tasks fit between them.
+//
+// A task takes all slices of a block where the level has `many` blocks or more:
+// two an SM (24^3 of order 2, forward and backward sweep with matvec rows: 1139
+// and 2830 us; with four 1140 and 2938, with one 1164 and 2811, never 1430 and
+// 3145; 12^3: 260 and 491, 250 and 495, 296 and 523, 250 and 495).
+static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& lev, int scale, int many, KeyedTasks& keyed) {
+    // blocks per level: inv(D) by the row's, entries by the parent's
+    std::vector<int> dlev, elev;
+    for (int pr = 0; pr < (int)P.prow_b.size(); ++pr) {
+        auto add = [](std::vector<int>& v, int l, int n) {
+            if ((int)v.size() <= l) v.resize(l + 1, 0);
+            v[l] += n;
+        };
+        add(dlev, lev[pr], 1);
+        for (const auto& en : (fwd ? P.lo : P.up)[pr]) add(elev, lev[en.parent], 1);
+    }
+    const int np = (int)P.prow_b.size();
+    const std::vector<uint8_t>& whole = fwd ? P.whole_f : P.whole_b;
+    std::vector<int> first(np + 1, 0);
+    for (int pr = 0; pr < np; ++pr) first[pr + 1] = first[pr] + (int)(fwd ? P.lo : P.up)[pr].size();
+    for (int32_t pr : fwd ? P.fwd_rows : P.bwd_rows) {
+        const auto& ents = (fwd ? P.lo : P.up)[pr];
+        const int b = P.prow_b[pr], ns = sweep_slices(b), ne = (int)ents.size();
+        StreamTask t{};
+        t.row = pr;
+        t.b = b;
+        t.zrow = P.z_off[pr];
+        t.vrow = P.v_off[pr];
+        t.q0 = first[pr];
+        t.q1 = first[pr + 1];
+        t.wait = -1;
+        t.par = pr;
+        t.pb = b;
+        if (whole[pr]) {
+            t.code = SW_ROW;
+            for (const auto& en : ents) t.cols += en.nc;
+            t.off = fwd ? (ne ? ents[0].l_off : 0) : P.dinv_off[pr];
+            t.out = t.rbase = fwd ? 0 : P.base_u[pr];
+            t.nall = ne ? 1 : 0;
+            t.src = !fwd && P.lo[pr].empty();
+            keyed.add(scale * (2 * lev[pr] - 1), t);
+            continue;
+        }
+        const int dstep = dlev[lev[pr]] >= many ? ns : 1;
+        if (!fwd)
+            for (int s = 0; s < ns; s += dstep) {
+                StreamTask u = t;
+                u.nc = b;
+                u.s0 = s;
+                u.nsl = dstep;
+                const int c0 = b * s / ns;
+                u.code = SW_DIAG;
+                u.cols = b * (s + dstep) / ns - c0;
+                u.off = P.dinv_off[pr] + (int64_t)c0 * b;
+                u.out = P.base_d[pr] + (int64_t)s * b;
+                u.rbase = P.base_d[pr];
+                u.nall = ns;
+                u.wait = ne ? ne * ns : -1;
+                u.npart = ne * ns;
+                // z_r = v_r in a row without lower entries
+                u.src = P.lo[pr].empty();
+                u.seg = (u.src ? t.vrow : t.zrow) + c0;
+                u.pseg = P.base_u[pr] + c0;
+                keyed.add(scale * (2 * lev[pr] - 1), u);
+            }
+        for (int e = 0; e < ne; ++e) {
+            const int step = elev[lev[ents[e].parent]] >= many ? ns : 1;
+            for (int s = 0; s < ns; s += step) {
+                StreamTask u = t;
+                u.nc = ents[e].nc;
+                u.s0 = s;
+                u.nsl = step;
+                const int q = ents[e].parent, nc = ents[e].nc, c0 = nc * s / ns, nq = (int)(fwd ? P.lo : P.up)[q].size();
+                const int nsq = sweep_slices(nc);
+                u.code = SW_ENTRY;
+                u.cols = nc * (s + step) / ns - c0;
+                u.off = (fwd ? ents[e].l_off : ents[e].a_off) + (int64_t)c0 * b;
+                u.rbase = fwd ? P.base_f[pr] : P.base_u[pr];
+                u.out = u.rbase + (int64_t)(e * ns + s) * b;
+                u.nall = ne * ns;
+                u.par = q;
+                u.pb = nc;
+                if (whole[q]) {
+                    u.wait = 0;
+                    u.src = 0;
+                    u.seg = P.z_off[q] + c0;
+                } else if (fwd) {
+                    u.wait = nq ? nq * nsq : -1;
+                    u.npart = nq * nsq;
+                    u.src = 1;
+                    u.seg = P.v_off[q] + c0;
+                    u.pseg = P.base_f[q] + c0;
+                } else {
+                    u.wait = nsq;
+                    u.npart = nsq;
+                    u.src = 2;
+                    u.pseg = P.base_d[q] + c0;
+                }
+                keyed.add(scale * (2 * lev[q]), u);
+            }
+        }
+        if (fwd && ne == 0) {
+            // z_r = v_r for whoever reads it (the backward sweep): a slice of no columns
+            StreamTask u = t;
+            u.code = SW_ENTRY;
+            u.rbase = u.out = P.base_f[pr];
+            u.nall = 1;
+            u.nsl = 1;
+            keyed.add(-scale, u);
+        }
+    }
+}
+
 // Levels, LD slots, GEMM tasks, device upload.
 static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluProgram& P) {
     const int np = (int)P.prow_b.size();
@@ -1307,11 +1492,8 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
     // task-split sweeps: one task per entry, combine-only tasks for rows
     // without entries; hand-out order by the level of the parent row
     {
-        // with_diag: the streamed backward sweep's list, where each row also
-        // has an inv(D) task (entry -2) keyed between the U tasks it waits for
-        // (keys 2*level(parent) < 2*level(row)) and its children's U tasks
         auto build_tasks = [&](bool fwd, std::vector<int32_t>& trow, std::vector<int32_t>& tent,
-                               std::vector<int64_t>& poff, int64_t& psize, bool with_diag = false) {
+                               std::vector<int64_t>& poff, int64_t& psize) {
             const std::vector<int32_t>& order = fwd ? P.fwd_rows : P.bwd_rows;
             const std::vector<int>& lev = fwd ? lf : lb;
             std::vector<std::pair<int, std::pair<int32_t, int32_t>>> keyed;
@@ -1326,10 +1508,8 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
             }
             for (int32_t pr : order) {
                 const auto& ents = fwd ? P.lo[pr] : P.up[pr];
-                const int sc = with_diag ? 2 : 1;
-                if (with_diag) keyed.push_back({2 * lev[pr] - 1, {pr, -2}});
-                else if (ents.empty()) keyed.push_back({-1, {pr, -1}});
-                for (size_t e = 0; e < ents.size(); ++e) keyed.push_back({sc * lev[ents[e].parent], {pr, first[pr] + (int32_t)e}});
+                if (ents.empty()) keyed.push_back({-1, {pr, -1}});
+                for (size_t e = 0; e < ents.size(); ++e) keyed.push_back({lev[ents[e].parent], {pr, first[pr] + (int32_t)e}});
             }
             std::stable_sort(keyed.begin(), keyed.end(), [](const auto& a, const auto& c) { return a.first < c.first; });
             trow.clear();
@@ -1349,10 +1529,6 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
         if ((st0 = upload_array(ctx, P.d_tb_row, tr)) || (st0 = upload_array(ctx, P.d_tb_ent, te)) ||
             (st0 = upload_array(ctx, P.d_poff_b, po)))
             return st0;
-        int64_t psb = 0;
-        build_tasks(false, tr, te, po, psb, true);
-        P.ntask_sb = (int)tr.size();
-        if ((st0 = upload_array(ctx, P.d_sb_row, tr)) || (st0 = upload_array(ctx, P.d_sb_ent, te))) return st0;
     }
     // LD slots: per programme row [inv(D)][L_1][L_2]...
     P.dinv_off.assign(np, 0);
@@ -1364,6 +1540,18 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
         for (auto& en : P.lo[pr]) { en.l_off = ld; ld += (int64_t)b * en.nc; }
     }
     P.ld_size = ld;
+    // streamed sweeps: the tasks in key order
+    stream_layout(P);
+    for (int fwd = 1; fwd >= 0; --fwd) {
+        KeyedTasks keyed(-1);
+        for (int pass = 0; pass < 2; ++pass) {
+            stream_tasks(P, fwd != 0, fwd ? lf : lb, 1, 2 * ctx->nsm, keyed);
+            if (pass == 0) keyed.place();
+        }
+        int st0;
+        if ((st0 = upload_array(ctx, fwd ? P.d_sf_task : P.d_sb_task, keyed.task))) return st0;
+        (fwd ? P.ntask_sf : P.ntask_sb) = (int)keyed.task.size();
+    }
     // flatten entry lists
     std::vector<int32_t> lo_ptr(np + 1, 0), up_ptr(np + 1, 0), lo_par, up_par, lo_nc, up_nc;
     std::vector<int64_t> lo_L, up_U;
@@ -1489,8 +1677,8 @@ void chidg::release_program(IluProgram& P) {
     for (Buffer* b : {&P.d_prow_b, &P.d_prow_elem, &P.d_v_off, &P.d_z_off, &P.d_dinv_off, &P.d_lo_ptr, &P.d_lo_L,
                       &P.d_lo_par, &P.d_lo_nc, &P.d_up_ptr, &P.d_up_U, &P.d_up_par, &P.d_up_nc, &P.d_fwd_rows,
                       &P.d_bwd_rows, &P.d_ltasks, &P.d_lpairs, &P.d_stasks, &P.d_spairs, &P.d_ltask_of, &P.d_tf_row, &P.d_tf_ent,
-                      &P.d_tb_row, &P.d_tb_ent, &P.d_poff_f, &P.d_poff_b, &P.d_sb_row, &P.d_sb_ent, &P.d_asm_ptr,
-                      &P.d_asm_src, &P.d_asm_r0, &P.d_asm_c0, &P.d_asm_nr, &P.d_asm_nc, &P.d_bmv_row, &P.d_bmv_ent,
+                      &P.d_tb_row, &P.d_tb_ent, &P.d_poff_f, &P.d_poff_b, &P.d_sf_task, &P.d_sb_task, &P.d_asm_ptr,
+                      &P.d_asm_src, &P.d_asm_r0, &P.d_asm_c0, &P.d_asm_nr, &P.d_asm_nc, &P.d_bmv_task,
                       &P.d_col_prow, &P.d_mv_skip})
         release(*b);
     P.bmv_uid = -1;
@@ -1511,7 +1699,7 @@ static int build_programme(chidg_gpu_precon* M, chidg_gpu_matrix* A) {
                                            : build_ilu0(S, M->kind == CHIDG_PRECON_JACOBI, M->P, err);
     if (st) { release_program(M->P); return fail(ctx, st, err); }
     if ((st = finalize_program(ctx, S, M->P))) { release_program(M->P); return st; }
-    const size_t sync_bytes = sizeof(unsigned) * (2 + 4 * (size_t)M->P.nprow);
+    const size_t sync_bytes = sizeof(unsigned) * (2 + 5 * (size_t)M->P.nprow);
     if ((st = ensure(ctx, M->sync, sync_bytes))) { release_program(M->P); return st; }
     cudaMemsetAsync(M->sync.ptr, 0, sync_bytes, ctx->stream);
     M->built_transposed = A->transposed && !own;
@@ -1754,7 +1942,7 @@ extern "C" int chidg_gpu_precon_update(chidg_gpu_precon* M, chidg_gpu_matrix* A,
     // fresh task counters for the task-split sweeps (a sweep cut short by an
     // error would otherwise leave them out of step)
     if (M->sync.ptr)
-        cudaMemsetAsync((unsigned*)M->sync.ptr + 2 + P.nprow, 0, sizeof(unsigned) * 3 * (size_t)P.nprow, ctx->stream);
+        cudaMemsetAsync((unsigned*)M->sync.ptr + 2 + P.nprow, 0, sizeof(unsigned) * 4 * (size_t)P.nprow, ctx->stream);
     if ((precision == CHIDG_GPU_MIXED_FP32 || precision == CHIDG_GPU_MIXED_BF16) && !P.assembled) {
         // the inner solves only read FP32 / BF16 factors: compute them in FP32
         if ((st = factor_fp32(M, A, precision))) return st;
@@ -1884,7 +2072,7 @@ static int dataflow_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const
     const int grid = M->sf_grid[variant];
     unsigned* counters = (unsigned*)M->sync.ptr;
     SweepSync S{counters, counters + 2, 0u, (int*)(ctx->d_scal + kSlotStatus), kSpinLimit};
-    cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned), ctx->stream);
+    cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned) * (2 + 5 * (size_t)P.nprow), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sweep counters");
     int ph = prof_begin(ctx, sizeof(TV) == 8 ? kProfIluForward : kProfIlu32);
     S.epoch = ++M->epoch;
@@ -1935,7 +2123,7 @@ static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV*
     unsigned* sync = (unsigned*)M->sync.ptr;
     unsigned* flags = sync + 2;
     SweepSync S{sync, flags, 0u, (int*)(ctx->d_scal + kSlotStatus), kSpinLimit};
-    cudaError_t e = cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), ctx->stream);
+    cudaError_t e = cudaMemsetAsync(sync, 0, sizeof(unsigned) * (2 + 5 * (size_t)P.nprow), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sweep counters");
     int ph = prof_begin(ctx, sizeof(TV) == 8 ? kProfIluForward : kProfIlu32);
     S.epoch = ++M->epoch;
@@ -1959,11 +2147,17 @@ static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV*
 }
 
 // The shape table: per kernel kind, block-size class and value width.
-// Defaults: 8 consumer warps, 2 stages of 24 KB; the backward sweep with the
-// matvec rows 2 stages of 20 KB, so that its wider staged segment still lets
-// 4 CTAs share an SM (measured: 3.62 against 3.80 ms at 24^3 P2 with 24 KB
-// and 3 CTAs).  CHIDG_STREAM_SHAPE="warps,stages,kbytes" overrides the
-// sweeps' defaults (comparison runs).
+// Defaults of the sweeps: 8 consumer warps and two stages (four where every row
+// is one task of few bytes) of 24 KB forward and 26 KB backward, which slices fill
+// evenly: 45 columns of 135 rows are three chunks of the one, so that four CTAs
+// share an SM, and two of the other; 40 columns of 320 rows five and four.  The
+// stage size is the same in every class, so that a row is chunked, and sums, the
+// same whatever the largest block beside it.  Forward sweep and backward sweep
+// with matvec rows within FP64 solves, us, 24 / 26 KB: 24^3 of order 2 1137 / 1207
+// and 3229 / 2957, 12^3 250 / 240 and 555 / 496, 9 x 8 x 10 of order 3 346 / 362
+// and 882 / 851; 20 KB 1160, 249, 357 and 2941, 527, 950.
+// CHIDG_STREAM_SHAPE="warps,stages,kbytes" overrides the sweeps' defaults
+// (comparison runs).
 namespace {
 std::mutex g_shape_mu;
 StreamShape g_shape[kShapeKinds][kShapeClasses][3];
@@ -1971,17 +2165,19 @@ bool g_shape_init = false;
 int width_slot(int esz) { return esz >= 8 ? 0 : esz == 4 ? 1 : 2; }
 void init_shapes() {
     StreamShape sweep;
+    bool given = false;
     if (const char* e = std::getenv("CHIDG_STREAM_SHAPE")) {
         int cw = 0, ns = 0, kb = 0;
         if (std::sscanf(e, "%d,%d,%d", &cw, &ns, &kb) == 3 && (cw == 4 || cw == 8 || cw == 16) && ns >= 2 &&
             ns <= SS_MAX_STAGES && kb >= 2 && kb <= 96)
-            sweep = StreamShape{cw, ns, kb * 1024};
+            { sweep = StreamShape{cw, ns, kb * 1024}; given = true; }
     }
     for (int c = 0; c < kShapeClasses; ++c)
         for (int w = 0; w < 3; ++w) {
-            g_shape[kShapeForward][c][w] = sweep;
-            g_shape[kShapeBackward][c][w] = sweep;
-            g_shape[kShapeBackwardMv][c][w] = StreamShape{8, 2, 20 * 1024};
+            const StreamShape def{8, c == 0 ? 4 : 2, 26 * 1024};
+            g_shape[kShapeForward][c][w] = given ? sweep : StreamShape{8, def.nstage, 24 * 1024};
+            g_shape[kShapeBackward][c][w] = given ? sweep : def;
+            g_shape[kShapeBackwardMv][c][w] = def;
             g_shape[kShapeMatvec][c][w] = StreamShape{8, 2, 24 * 1024};
         }
     g_shape_init = true;
@@ -2022,7 +2218,7 @@ static int stream_launch(chidg_gpu_precon* M, const TL* LD, const TU* U, StreamT
                          int mv_cols = 0) {
     chidg_gpu_ctx* ctx = M->ctx;
     using ACC = typename AccOf<TV>::type;
-    const int xcols = std::max(M->P.max_b, mv_cols);    // the widest segment staged in shared memory
+    const int xcols = std::max({M->P.max_b, M->P.max_row_task_cols, mv_cols});    // the widest segment staged in shared memory
     // a stage must hold one column of the widest block (plus the 16-byte rounding)
     if ((size_t)sh.stage_bytes < (size_t)M->P.max_b * std::max(sizeof(TL), sizeof(TU)) + 16 ||
         (MV && (size_t)sh.stage_bytes < (size_t)M->P.max_b * sizeof(TA) + 16))
@@ -2044,24 +2240,17 @@ static int stream_launch(chidg_gpu_precon* M, const TL* LD, const TU* U, StreamT
 }
 
 // Task list of the backward sweep with the matvec rows of A in it: the
-// streamed backward sweep's tasks in their order (the keys of finalize_program,
-// scaled by 4), and for every matrix row r a task (r, -3) keyed after the
-// inv(D) task of the last row its columns read, `lag` levels later, so that
+// streamed backward sweep's tasks in their order (the keys of stream_tasks,
+// scaled by 4), and for every matrix row r a task (r, SW_MATVEC) keyed after the
+// last tasks of the last row its columns read, `lag` levels later, so that
 // when a CTA takes it the rows it waits for are most likely published.  A
 // matvec task waits only for tasks with smaller tickets (deadlock freedom as
 // for the sweep).  Needs programme rows == matrix rows (ILU0, Jacobi).
 static int build_bwd_mv_tasks(chidg_gpu_precon* M, const chidg_gpu_matrix* A, int lag) {
     IluProgram& P = M->P;
     if (P.bmv_uid == A->uid && P.bmv_lag == lag) return CHIDG_GPU_OK;
-    const int np = P.nprow;
-    std::vector<int> first(np + 1, 0);
-    for (int pr = 0; pr < np; ++pr) first[pr + 1] = first[pr] + (int)P.up[pr].size();
-    std::vector<std::pair<int64_t, std::pair<int32_t, int32_t>>> keyed;
-    for (int32_t pr : P.bwd_rows) {
-        keyed.push_back({4LL * (2 * P.lb[pr] - 1), {pr, -2}});
-        for (size_t e = 0; e < P.up[pr].size(); ++e)
-            keyed.push_back({4LL * (2 * P.lb[P.up[pr][e].parent]), {pr, first[pr] + (int32_t)e}});
-    }
+    std::vector<std::pair<int, StreamTask>> rows;
+    rows.reserve((size_t)A->nrow);
     std::vector<int32_t> col_prow;
     col_prow.reserve(A->nblk);
     // the matrix blocks that are the sweep's U blocks (same values, same
@@ -2085,19 +2274,27 @@ static int build_bwd_mv_tasks(chidg_gpu_precon* M, const chidg_gpu_matrix* A, in
             skip.push_back(u);
         }
         if (matched != (int)P.up[r].size()) reuse = false;
-        keyed.push_back({4LL * (last + 2 * lag) + 2, {r, -3}});
+        StreamTask t{};
+        t.row = r;
+        t.code = SW_MATVEC;
+        t.b = P.prow_b[r];
+        t.rbase = P.base_u[r];
+        t.nall = P.up[r].empty() ? 0 : P.whole_b[r] ? 1 : (int)P.up[r].size() * sweep_slices(t.b);
+        t.wait = -1;
+        rows.push_back({4 * (last + 2 * lag) + 2, t});
     }
-    std::stable_sort(keyed.begin(), keyed.end(), [](const auto& a, const auto& c) { return a.first < c.first; });
-    std::vector<int32_t> tr, te;
-    tr.reserve(keyed.size());
-    te.reserve(keyed.size());
-    for (auto& k : keyed) { tr.push_back(k.second.first); te.push_back(k.second.second); }
+    KeyedTasks keyed(-4);
+    for (int pass = 0; pass < 2; ++pass) {
+        stream_tasks(P, false, P.lb, 4, 2 * M->ctx->nsm, keyed);
+        for (const auto& r : rows) keyed.add(r.first, r.second);
+        if (pass == 0) keyed.place();
+    }
     int st;
-    if ((st = upload_array(M->ctx, P.d_bmv_row, tr)) || (st = upload_array(M->ctx, P.d_bmv_ent, te)) ||
-        (st = upload_array(M->ctx, P.d_col_prow, col_prow)) || (st = upload_array(M->ctx, P.d_mv_skip, skip)))
+    if ((st = upload_array(M->ctx, P.d_bmv_task, keyed.task)) || (st = upload_array(M->ctx, P.d_col_prow, col_prow)) ||
+        (st = upload_array(M->ctx, P.d_mv_skip, skip)))
         return st;
     P.bmv_reuse = reuse;
-    P.ntask_bmv = (int)tr.size();
+    P.ntask_bmv = (int)keyed.task.size();
     P.bmv_uid = A->uid;
     P.bmv_lag = lag;
     return CHIDG_GPU_OK;
@@ -2144,38 +2341,25 @@ static int stream_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const T
     const StreamShape sh = stream_shape_for(kShapeForward, P.max_b, esz);
     const StreamShape shb = stream_shape_for(F ? kShapeBackwardMv : kShapeBackward, P.max_b, esz);
     Buffer& pb = (sizeof(ACC) == 8) ? M->part64 : M->part32;
-    int st = ensure(ctx, pb, sizeof(ACC) * (size_t)std::max<int64_t>(1, std::max(P.part_f, P.part_b)));
+    int st = ensure(ctx, pb, sizeof(ACC) * (size_t)P.part_s);
     if (st) return st;
+    // tickets, flags and counts start at zero in every call (also when it is
+    // replayed from a graph); a flag is set to a value no host epoch reaches
+    constexpr unsigned kStreamEpoch = 0xF0000001u;
     unsigned* sync = (unsigned*)M->sync.ptr;
-    unsigned* flags = sync + 2;
-    SweepSync S{sync, flags, 0u, (int*)(ctx->d_scal + kSlotStatus), kSpinLimit};
-    cudaError_t e = cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), ctx->stream);
+    unsigned* rowsync = sync + 2;
+    const size_t np = (size_t)P.nprow;
+    SweepSync S{sync, rowsync, kStreamEpoch, (int*)(ctx->d_scal + kSlotStatus), kSpinLimit};
+    cudaError_t e = cudaMemsetAsync(sync, 0, sizeof(unsigned) * (2 + 5 * np), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sweep counters");
     int ph = prof_begin(ctx, sizeof(TV) == 8 ? kProfIluForward : kProfIlu32);
-    // inside a captured sequence: clear the row flags (and the backward
-    // sweep's ready flags) in the sequence itself and publish fixed epochs,
-    // which no host epoch reaches
-    constexpr unsigned kGraphEpochF = 0xF0000001u, kGraphEpochB = 0xF0000002u;
-    auto clear_flags = [&](bool backward) -> int {
-        cudaError_t e2 = cudaMemsetAsync(flags, 0, sizeof(unsigned) * (size_t)P.nprow, ctx->stream);
-        if (e2 == cudaSuccess && backward)
-            e2 = cudaMemsetAsync(flags + 3 * P.nprow, 0, sizeof(unsigned) * (size_t)P.nprow, ctx->stream);
-        return e2 == cudaSuccess ? CHIDG_GPU_OK : cuda_fail(ctx, e2, "sweep flags");
-    };
-    if (which & 1) {
-        if (M->graph_safe) {
-            if ((st = clear_flags(false))) return st;
-            S.epoch = kGraphEpochF;
-        } else {
-            S.epoch = ++M->epoch;
-        }
-        S.counter = sync;
-        StreamTasks Tf{(const int32_t*)P.d_tf_row.ptr, (const int32_t*)P.d_tf_ent.ptr, (const int64_t*)P.d_poff_f.ptr,
-                       flags + P.nprow, flags + 3 * P.nprow};
+    // without lower entries (Jacobi, HB) the backward sweep reads v itself
+    if ((which & 1) && !P.no_lower) {
+        const StreamTasks Tf{(const StreamTask*)P.d_sf_task.ptr, rowsync + np, nullptr};
         switch (sh.cw) {
-            case 16: st = stream_launch<TL, TU, TV, true, 16>(M, LD, U, Tf, P.ntask_f, v, zx, pb.ptr, S, sh, variant); break;
-            case 4: st = stream_launch<TL, TU, TV, true, 4>(M, LD, U, Tf, P.ntask_f, v, zx, pb.ptr, S, sh, variant); break;
-            default: st = stream_launch<TL, TU, TV, true, 8>(M, LD, U, Tf, P.ntask_f, v, zx, pb.ptr, S, sh, variant);
+            case 16: st = stream_launch<TL, TU, TV, true, 16>(M, LD, U, Tf, P.ntask_sf, v, zx, pb.ptr, S, sh, variant); break;
+            case 4: st = stream_launch<TL, TU, TV, true, 4>(M, LD, U, Tf, P.ntask_sf, v, zx, pb.ptr, S, sh, variant); break;
+            default: st = stream_launch<TL, TU, TV, true, 8>(M, LD, U, Tf, P.ntask_sf, v, zx, pb.ptr, S, sh, variant);
         }
         if (st) return st;
     }
@@ -2187,16 +2371,10 @@ static int stream_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const T
         prof_end(ctx, ph);
         ph = prof_begin(ctx, F ? kProfIluBackwardMv : kProfIluBackward);
     }
-    if (M->graph_safe) {
-        if ((st = clear_flags(true))) return st;
-        S.epoch = kGraphEpochB;
-    } else {
-        S.epoch = ++M->epoch;
-    }
+    S.flags = rowsync + 2 * np;
     S.counter = sync + 1;
     if (F) {
-        StreamTasks Tm{(const int32_t*)P.d_bmv_row.ptr, (const int32_t*)P.d_bmv_ent.ptr, (const int64_t*)P.d_poff_b.ptr,
-                       flags + 2 * P.nprow, flags + 3 * P.nprow};
+        const StreamTasks Tm{(const StreamTask*)P.d_bmv_task.ptr, rowsync + 3 * np, rowsync + 4 * np};
         // the sweep's U partials stand for the matvec's U blocks only when
         // the sweep reads the matvec's own values
         FusedMv<TA, TV> Fr = *F;
@@ -2213,8 +2391,7 @@ static int stream_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const T
         prof_end(ctx, ph);
         return CHIDG_GPU_OK;
     }
-    StreamTasks Tb{(const int32_t*)P.d_sb_row.ptr, (const int32_t*)P.d_sb_ent.ptr, (const int64_t*)P.d_poff_b.ptr,
-                   flags + 2 * P.nprow, flags + 3 * P.nprow};
+    const StreamTasks Tb{(const StreamTask*)P.d_sb_task.ptr, rowsync + 3 * np, rowsync + 4 * np};
     switch (shb.cw) {
         case 16: st = stream_launch<TL, TU, TV, false, 16>(M, LD, U, Tb, P.ntask_sb, v, zx, pb.ptr, S, shb, variant); break;
         case 4: st = stream_launch<TL, TU, TV, false, 4>(M, LD, U, Tb, P.ntask_sb, v, zx, pb.ptr, S, shb, variant); break;
@@ -2464,13 +2641,13 @@ __global__ void k_fill32(float* x, int64_t n, float v) {
 }  // namespace
 
 // Candidate shapes: 4, 8 or 16 consumer warps; 2 to 4 stages of 8 to 48 KB
-// (ring at most 96 KB); a stage holds at least one column of the widest block.
+// (ring at most 104 KB); a stage holds at least one column of the widest block.
 static std::vector<StreamShape> shape_candidates(int max_b, int esz) {
     std::vector<StreamShape> out;
     for (int cw : {4, 8, 16})
         for (int ns : {2, 3, 4})
-            for (int kb : {8, 12, 16, 20, 24, 32, 40, 48}) {
-                if (ns * kb > 96) continue;
+            for (int kb : {8, 12, 16, 20, 24, 25, 26, 32, 40, 48}) {
+                if (ns * kb > 104) continue;
                 if ((size_t)kb * 1024 < (size_t)max_b * esz + 16) continue;
                 out.push_back(StreamShape{cw, ns, kb * 1024});
             }

@@ -71,15 +71,22 @@ struct IluProgram {
     int ntask_f = 0, ntask_b = 0;
     int64_t part_f = 0, part_b = 0;            // scratch sizes (values)
     Buffer d_tf_row, d_tf_ent, d_tb_row, d_tb_ent, d_poff_f, d_poff_b;
-    int ntask_sb = 0;                          // streamed backward sweep: U tasks + inv(D) tasks
-    Buffer d_sb_row, d_sb_ent;
+    // streamed sweeps: tasks (StreamTask), partial sums (the two sweeps use the
+    // same scratch), the first partials of every row's entries and of inv(D)
+    int ntask_sf = 0, ntask_sb = 0;
+    int64_t part_s = 0;
+    int max_row_task_cols = 0;                 // widest segment a one-task row stages
+    std::vector<uint8_t> whole_f, whole_b;     // rows that are one task
+    bool no_lower = false;                     // no row has lower entries: the streamed forward sweep is left out
+    std::vector<int64_t> base_f, base_u, base_d;
+    Buffer d_sf_task, d_sb_task;
     std::vector<int> lb;                       // backward dependency level of every programme row
-    // streamed backward sweep with the following matvec's rows (entry -3),
+    // streamed backward sweep with the following matvec's rows (SW_MATVEC),
     // built for one matrix structure (bmv_uid) on first use
     int ntask_bmv = 0, bmv_lag = -1;
     int64_t bmv_uid = -1;
     bool bmv_reuse = false;                    // every U entry is a block of its matrix row (d_mv_skip)
-    Buffer d_bmv_row, d_bmv_ent, d_col_prow, d_mv_skip;
+    Buffer d_bmv_task, d_col_prow, d_mv_skip;
     // rows whose D is assembled from several blocks of A (precon_HB) instead
     // of starting from one diagonal block: pieces per row, placed at (r0, c0)
     bool assembled = false;
@@ -211,15 +218,11 @@ struct chidg_gpu_precon {
     chidg::IluProgram P;
     chidg::Buffer LD, LD32, LD16, zx, zx32, piv_scratch;
     int schedule = CHIDG_SCHED_STREAM;     // sweep schedule (TASKS for blocks over 1024 rows)
-    chidg::Buffer sync;                    // [2 counters][flags][forward row counts][backward row counts]
+    chidg::Buffer sync;                    // [2 tickets] and five words a row: flags and counts of the sweeps
     chidg::Buffer part64, part32;          // task-split sweep partials (FP64 / low precision)
     unsigned epoch = 0;
     int sf_grid[3] = {0, 0, 0};            // resident CTAs of the dataflow sweep per vector type
     int tk_grid[4] = {0, 0, 0, 0};         // resident CTAs of the task-split sweep per variant
-    // the sweeps are being captured into a CUDA graph: each sweep clears its
-    // row flags and publishes with a fixed epoch, so that every replay starts
-    // from cleared flags (a host epoch would be frozen into the graph)
-    bool graph_safe = false;
 };
 
 namespace chidg {

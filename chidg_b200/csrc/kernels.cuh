@@ -1091,7 +1091,7 @@ __global__ void k_seg_mdot(const int64_t* __restrict__ cstart, int nchunk, const
                            const T* __restrict__ y, int64_t ystride, int nq, double* __restrict__ partial,
                            const int32_t* __restrict__ csys = nullptr, const int32_t* __restrict__ mask = nullptr) {
     // eight vectors per pass over the chunk of x, each sum formed in the
-    // order of a pass per vector (as k_mdot_partial)
+    // order of a pass per vector (as k_mdot)
     constexpr int QG = 8;
     __shared__ double scratch[QG][32];
     const int c = blockIdx.x;
@@ -1224,9 +1224,9 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
 __device__ __forceinline__ bool wait_flag(const unsigned* flags, int row, unsigned epoch, long long limit) {
     if (ld_acquire(flags + row) == epoch) return true;
     const long long t0 = clock64();
-    while (ld_acquire(flags + row) != epoch) {
+    for (int k = 0; ld_acquire(flags + row) != epoch; ++k) {
         if (clock64() - t0 > limit) return false;
-        __nanosleep(64);
+        if (k > 16) __nanosleep(32);
     }
     return true;
 }

@@ -78,8 +78,8 @@ __global__ void __launch_bounds__(32 * CW + 32)
                 // a frozen system's row: one empty chunk, nothing read or written
                 if (!mbar_wait(empty + stage, phase ^ 1u, spin_limit)) atomicExch(status, 1);
                 StreamMeta m;
-                m.task = row; m.pr = row; m.q = 0; m.chunk = 0; m.nchunk = 1;
-                m.col0 = 0; m.ncols = 0; m.shift = 0; m.skip = 1;
+                m.task = row; m.chunk = 0; m.nchunk = 1;
+                m.col0 = 0; m.ncols = 0; m.shift = 0; m.skip = 1; m.end = 0;
                 meta[stage] = m;
                 mbar_arrive(full + stage);
                 if (++stage == nstage) { stage = 0; phase ^= 1u; }
@@ -96,8 +96,8 @@ __global__ void __launch_bounds__(32 * CW + 32)
             for (int ch = 0; ch < nchunk; ++ch) {
                 if (!mbar_wait(empty + stage, phase ^ 1u, spin_limit)) atomicExch(status, 1);
                 StreamMeta m;
-                m.task = row; m.pr = row; m.q = 0; m.chunk = ch; m.nchunk = nchunk;
-                m.skip = 0;
+                m.task = row; m.chunk = ch; m.nchunk = nchunk;
+                m.skip = 0; m.end = 0;
                 m.col0 = ch * kc;
                 m.ncols = cols > 0 ? min(kc, cols - ch * kc) : 0;
                 m.shift = 0;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(32 * CW + 32)
             continue;
         }
         if (m.chunk == 0) {
-            row = m.pr;
+            row = m.task;
             b = R.row_b[row];
             if (b <= NC) { G = NC / b; r = ctid % b; g = ctid / b; }
             else { G = 1; r = ctid; g = 0; }

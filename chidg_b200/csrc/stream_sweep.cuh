@@ -1,32 +1,60 @@
 // ILU programme: streamed task sweeps (CHIDG_SCHED_STREAM).
 //
-// The work of one triangular sweep is the task list of the task-split sweep
-// (one block product per task, handed out in topological order of the parent
-// rows), executed by persistent CTAs (several per SM, so that several tasks
-// are in flight on each SM) with a producer/consumer split:
+// The work of one triangular sweep is a list of tasks (StreamTask), handed out
+// in topological order of the rows they wait for and executed by persistent
+// CTAs (several per SM, so that several tasks are in flight on each SM) with a
+// producer/consumer split:
 //
 //   producer (one lane of the last warp)  takes a ticket, and copies the task's
-//       block column-chunk by column-chunk into a ring of shared-memory stages
+//       blocks column-chunk by column-chunk into a ring of shared-memory stages
 //       with cp.async.bulk (completion counted on the stage's mbarrier).  The
 //       copy does not depend on the sweep's values, so it runs ahead of the
-//       dependency waits: the block is in shared memory when the parent row is
-//       published.
-//   consumers (the other warps)  wait (bounded) for the parent row, stage its
-//       segment of z, multiply the chunks as they land, release each stage, and
-//       at the last chunk publish the block's partial product.  The last task of
-//       a row to finish completes it.
+//       dependency waits: the chunks are in shared memory when the parent row
+//       is published.  The next ticket and its descriptor are fetched while
+//       the current task's chunks are posted.
+//   consumers (the other warps)  wait (bounded) for the parent rows, stage their
+//       segments of z, multiply the chunks as they land, release each stage, and
+//       at the task's last chunk publish its result.
 //
-// Backward sweep: the product with inv(D_r) is a task of its own (entry -2),
-// ordered after the row's U tasks and before its children's; it waits for
-// the row's partials to be complete (the `ready` flag set by the last U task),
-// adds them to z_r in entry order and multiplies by inv(D_r) streamed through
-// the same ring, so inv(D_r) is prefetched like every other block.
+// A sweep is a chain of rows (levels), and where a level holds few rows its
+// time is that of one hop: parent published, segment fetched, block
+// multiplied, row completed and published.  What is on that path is kept
+// short:
+//
+//   rows of at most SW_ROW_B equations (order 1 with five fields: 40) are one
+//       task with all their blocks, inv(D) included in the backward sweep: one
+//       flag a row, no partial sums through memory.
+//   larger blocks are cut into sweep_slices(b) slices of columns, a task each:
+//       135 columns are three slices of 49 KB, 320 columns eight of 102 KB; as
+//       one task (146 or 819 KB) most of a block was still to be streamed by
+//       one CTA when its parent was published.
+//       Where a level has slices enough to fill the chip, a task takes all of a
+//       block's slices one after another (the same sums, one wait).
+//   a slice leaves its partial sums and counts itself; nobody gathers them on
+//       the path: a task that needs the row adds the partials up itself, in
+//       order, while it stages them (forward: z_r = v_r - sum of the row's
+//       partials; backward: the slices of inv(D_r) stage z_r - sum of the U
+//       partials, and the row's children add up the partials of inv(D_r)).
+//       The last task of a row to finish writes z_r itself, for whoever reads it
+//       later.
+//   a task's indices come with its descriptor, not from dependent loads after
+//       the wait (an acquire leaves the SM's L1 without them).
+//
+// The cut depends on the row's own block size only, so a row sums in the same
+// order whatever matrix or batch it belongs to.
+//
+// Bound by the copies at 24^3 elements of order 2 (5.8 and 15.8 GB: 1.14 ms
+// forward, 2.83 ms backward with matvec rows; with whole blocks as tasks 1.20 and
+// 2.85) and by the hops in smaller boxes: 12^3 260 and 491 us (392 and 699), 9 x 8
+// x 10 of order 3 346 and 853 us (988 and 2054), 8^3 of order 1 64 and 101 us (103
+// and 160).
 //
 // Deadlock freedom: a task waits only for tasks with smaller tickets.  Each
 // CTA consumes its tasks in ticket order, and a producer posts a task's chunks
 // as soon as stages free, so the unfinished task with the smallest ticket can
-// always proceed.  Every wait (flags, mbarriers) is bounded; on a timeout the
-// sweep records status 1 and finishes with wrong values instead of hanging.
+// always proceed.  Every wait (flags, counts, mbarriers) is bounded; on a
+// timeout the sweep records status 1 and finishes with wrong values instead of
+// hanging.
 //
 // Bulk copies need 16-byte aligned source, destination and size: each chunk's
 // source is rounded down to 16 bytes (the element offset inside the stage is
@@ -41,14 +69,39 @@ namespace chidg {
 constexpr int SS_MAX_B = 1024;                              // rows per block
 constexpr int SS_MAX_STAGES = 8;
 constexpr int SS_MAX_NC = 512;                              // consumer threads (16 warps)
+constexpr int SS_BLKS = 32;                                 // blocks of a matvec row whose offsets are staged
+constexpr int SS_SLOTS = SS_MAX_STAGES + 3;                 // descriptors in flight: a ring of tasks, the one being finished and the next
+
+enum { SW_ENTRY = 0, SW_DIAG = 1, SW_ROW = 2, SW_MATVEC = 3 };   // slice of an entry, of inv(D); whole row; matvec row
+
+constexpr int SW_ROW_B = 64;      // rows of at most this size are one task (SW_ROW) ...
+constexpr int SW_ROW_COLS = 384;  // ... if their entries' columns fit the staged segment
+__host__ __device__ __forceinline__ int sweep_slices(int b) { return b <= SW_ROW_B ? 1 : b <= 160 ? 3 : 8; }
+
+// A task.  A slice's (or several adjacent slices') staged segment is base[seg + c] -/+ the sum of npart
+// partial vectors part[pseg + k * pb + c] (pb: their row's size), c < cols:
+// base is z (src 0), v (src 1) or nothing (src 2), the sum subtracted except
+// with src 2.  SW_ROW backward: the row's own z comes from z (src 0) or, without
+// lower entries, from v (src 1).
+struct alignas(16) StreamTask {
+    int32_t row, code, b, cols;     // programme row, its size, columns of the slice (SW_ROW forward: of all entries)
+    int64_t off;                    // the slice's first value in LD (forward, inv(D)) or A
+    int64_t zrow, vrow;             // the row's z and v
+    int64_t out, rbase;             // partials this task writes; first partials of its row (for the last task)
+    int64_t seg, pseg;
+    int32_t par, wait;              // the wait: < 0 none, 0 flag of par, n its count reaching n
+    int32_t npart, pb, src, nall;   // nall: tasks of the row (the last one completes it); SW_MATVEC, SW_ROW: U partial vectors of the row at rbase
+    int32_t q0, q1;                 // the row's entries
+    int32_t nc, s0, nsl;            // slices s0 .. s0 + nsl - 1 of nc columns
+};
 
 struct StreamMeta {
-    int task;      // ticket, -1 = end of the sweep for this CTA
-    int pr, q;     // programme row, entry (-1 combine-only, -2 backward diagonal)
+    int task;      // descriptor slot, -1 = end of the sweep for this CTA
     int chunk, nchunk;
     int col0, ncols;
     int shift;     // element offset of the chunk inside the stage
     int skip;      // the row's system is frozen: nothing is read, computed or written
+    int end;       // last chunk of a slice; SW_ROW backward: last chunk of the U blocks
 };
 
 // Rows of frozen systems in a batched solve (a system whose Arnoldi process
@@ -69,11 +122,9 @@ __device__ __forceinline__ bool row_frozen(const RowMask& mk, int row) {
 }
 
 struct StreamTasks {
-    const int32_t* task_row;
-    const int32_t* task_ent;
-    const int64_t* part_off;    // per entry: offset of its partial in the scratch vector
-    unsigned* row_count;        // per row: completed entry tasks, never reset (wraps by entry count)
-    unsigned* ready;            // backward: per row, epoch once all U partials are written
+    const StreamTask* task;
+    unsigned* count;            // per row: completed entry slices
+    unsigned* dcount;           // backward: per row, completed slices of inv(D)
 };
 
 // the row structure of a matrix whose rows' blocks are stored one after
@@ -96,12 +147,20 @@ __host__ __device__ constexpr size_t stream_xcap(int max_b) { return (size_t)((m
 // the row sums for the fused rows' sums of squares)
 __host__ __device__ constexpr size_t stream_smem_bytes(size_t acc_size, int stages, int stage_bytes, int max_b, int nc) {
     return (size_t)stages * stage_bytes + (stream_xcap(max_b) + nc) * acc_size + 32 * sizeof(double) +
-           2 * SS_MAX_STAGES * sizeof(uint64_t) + SS_MAX_STAGES * sizeof(StreamMeta) + 64;
+           2 * SS_MAX_STAGES * sizeof(uint64_t) + SS_MAX_STAGES * sizeof(StreamMeta) + SS_SLOTS * sizeof(StreamTask) + 64;
+}
+
+// columns a chunk of a strip of cols columns (b rows of esz bytes) takes: as
+// few chunks as the stage allows, of equal size
+__device__ __forceinline__ int chunk_cols(int cols, int b, int esz, int chunk_bytes) {
+    const int most = max(1, chunk_bytes / (b * esz));
+    const int n = (cols + most - 1) / most;
+    return n > 0 ? (cols + n - 1) / n : 1;
 }
 
 // The matvec that follows the backward sweep in FGMRES (w = A z_j,
 // type_fgmres.f90:175-189), run inside the backward sweep's launch: one task
-// per matrix row (entry -3), handed out after the sweep tasks that publish
+// per matrix row (SW_MATVEC), handed out after the sweep tasks that publish
 // the rows its columns read, so the rows' values stream while the sweep's
 // dependency chain waits.
 //
@@ -110,11 +169,10 @@ __host__ __device__ constexpr size_t stream_smem_bytes(size_t acc_size, int stag
 // precon_ILU0.f90:370-395), and z_j is final when they are formed.  With
 // `skip` set (the sweep's U blocks are the matvec's values, same type), the
 // matvec row streams only the blocks the sweep did not read -- the diagonal,
-// the lower blocks and any others -- and adds the row's U partials, in entry
-// order, to their product: y_r = (A_rr z_r + sum_lower A_rk z_k) + sum_U
-// part.  That drops the U blocks' second read (3/7 of the matrix on a hex
-// box).  Without `skip`, row r computes y_r exactly as k_matvec_stream does
-// (same chunks, same per-thread order).
+// the lower blocks and any others -- and adds the row's U partials, in order,
+// to their product: y_r = (A_rr z_r + sum_lower A_rk z_k) + sum_U part.  That
+// drops the U blocks' second read (3/7 of the matrix on a hex box).  Chunks
+// stay within a block.
 template <typename TA, typename TX>
 struct FusedMv {
     MatvecRowsView rows;         // the matrix rows (contiguous values per row)
@@ -231,10 +289,38 @@ __device__ __forceinline__ void stream_reduce(ACC* red, int b, int r, int g, int
     }
 }
 
+// s + n partial vectors (stride b) in order; eight loads go out together
+template <typename ACC>
+__device__ __forceinline__ ACC sum_partials_at(const ACC* p, int n, int b, ACC s) {
+    constexpr int U = 8;
+    for (int k0 = 0; k0 < n; k0 += U) {
+        ACC v[U];
+        #pragma unroll
+        for (int k = 0; k < U; ++k) v[k] = k0 + k < n ? ld_cg(p + (int64_t)(k0 + k) * b) : ACC(0);
+        #pragma unroll
+        for (int k = 0; k < U; ++k)
+            if (k0 + k < n) s += v[k];
+    }
+    return s;
+}
+// wait (one thread) until *p has reached target; false on timeout
+__device__ __forceinline__ bool wait_count(const unsigned* p, unsigned target, long long limit) {
+    if ((int)(ld_acquire(p) - target) >= 0) return true;
+    const long long t0 = clock64();
+    for (int k = 0; (int)(ld_acquire(p) - target) < 0; ++k) {
+        if (clock64() - t0 > limit) return false;
+        if (k > 16) __nanosleep(32);
+    }
+    return true;
+}
+__device__ __forceinline__ void red_release(unsigned* p, unsigned n) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(n) : "memory");
+}
+
 // CW consumer warps; `stages` stages of `stage_bytes` bytes each.  MV: the
-// backward sweep also runs the matvec rows of F (tasks with entry -3).
+// backward sweep also runs the matvec rows of F (tasks SW_MATVEC).
 template <typename TL, typename TU, typename TX, typename ACC, bool FORWARD, int CW, typename TA = double, bool MV = false>
-__global__ void __launch_bounds__(32 * CW + 32)
+__global__ void __launch_bounds__(32 * CW + 32, CW == 16 ? 2 : CW == 8 ? 4 : 7)   // CTAs an SM: what the rings leave room for
     k_ilu_stream(IluRows R, const TL* __restrict__ LD, const TU* __restrict__ Aval, StreamTasks T, int ntasks,
                  const TX* __restrict__ v, TX* __restrict__ zx, ACC* __restrict__ part, SweepSync S, int nstage,
                  int stage_bytes, int max_b, FusedMv<TA, TX> F, RowMask mask) {
@@ -244,13 +330,16 @@ __global__ void __launch_bounds__(32 * CW + 32)
     constexpr int RPT = (SS_MAX_B + NC - 1) / NC;
     extern __shared__ __align__(128) unsigned char ss_smem[];
     unsigned char* stages = ss_smem;
-    ACC* xs = reinterpret_cast<ACC*>(ss_smem + (size_t)nstage * stage_bytes);
-    ACC* red = xs + stream_xcap(max_b);          // G*b <= NC row sums
-    double* scratch = reinterpret_cast<double*>(red + NC);   // 32 doubles
+    StreamTask* slots = reinterpret_cast<StreamTask*>(ss_smem + (size_t)nstage * stage_bytes);
+    double* scratch = reinterpret_cast<double*>(slots + SS_SLOTS);   // 32 doubles
     uint64_t* full = reinterpret_cast<uint64_t*>(scratch + 32);
     uint64_t* empty = full + SS_MAX_STAGES;
-    StreamMeta* meta = reinterpret_cast<StreamMeta*>(empty + SS_MAX_STAGES);
+    ACC* xs = reinterpret_cast<ACC*>(empty + SS_MAX_STAGES);
+    ACC* red = xs + stream_xcap(max_b);          // G*b <= NC row sums
+    StreamMeta* meta = reinterpret_cast<StreamMeta*>(red + NC);
     __shared__ int s_last;
+    __shared__ int s_nc[SS_BLKS];                // SW_MATVEC: columns and x offsets (-1: not staged) of the row's blocks
+    __shared__ int64_t s_x[SS_BLKS];
     const int chunk_bytes = stage_bytes - 16;    // payload before rounding out to 16 bytes
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -266,115 +355,116 @@ __global__ void __launch_bounds__(32 * CW + 32)
     if (warp == CW) {
         // ------------------------------------------------------------ producer
         if (lane != 0) return;
-        int stage = 0;
+        int stage = 0, slot = 0;
         unsigned phase = 0;
-        for (;;) {
-            const unsigned t = atomicAdd(S.counter, 1u);
-            if (t >= (unsigned)ntasks) {
-                if (!mbar_wait(empty + stage, phase ^ 1u, S.spin_limit)) atomicExch(S.status, 1);
-                meta[stage].task = -1;
-                mbar_arrive(full + stage);
-                return;
-            }
-            const int pr = T.task_row[t], q = T.task_ent[t];
-            if (row_frozen(mask, pr)) {
+        unsigned t = atomicAdd(S.counter, 1u);
+        // descriptors live in shared memory; the next one's slot is free: the ring
+        // and the consumers hold fewer tasks than there are slots
+        if (t < (unsigned)ntasks) slots[0] = T.task[t];
+        while (t < (unsigned)ntasks) {
+            const StreamTask& d = slots[slot];
+            unsigned tn = 0;
+            const int b = d.b;
+            int ch = 0, nchunk = 0;
+            // columns [col0, col0 + ncols) of the staged segment times the strip at src
+            auto post = [&](const void* from, int col0, int ncols, int esz, int end, int skip) {
+                // the next ticket, its latency under the wait for the last
+                // chunk's stage: not earlier, or a long task would keep a
+                // short one waiting that another CTA could take
+                if (ch == nchunk - 1) tn = atomicAdd(S.counter, 1u);
                 if (!mbar_wait(empty + stage, phase ^ 1u, S.spin_limit)) atomicExch(S.status, 1);
                 StreamMeta m;
-                m.task = (int)t; m.pr = pr; m.q = q; m.chunk = 0; m.nchunk = 1;
-                m.col0 = 0; m.ncols = 0; m.shift = 0; m.skip = 1;
+                m.task = slot; m.chunk = ch; m.nchunk = nchunk;
+                m.col0 = col0; m.ncols = ncols; m.skip = skip; m.end = end;
+                const uintptr_t src = reinterpret_cast<uintptr_t>(from);
+                const uintptr_t a0 = src & ~(uintptr_t)15;
+                m.shift = ncols > 0 ? (int)(src - a0) / esz : 0;
                 meta[stage] = m;
-                mbar_arrive(full + stage);
-                if (++stage == nstage) { stage = 0; phase ^= 1u; }
-                continue;
-            }
-            int b = R.prow_b[pr];
-            const unsigned char* base = nullptr;
-            int cols = 0, esz = 1;
-            if (MV && q == -3) {
-                // matvec row pr: the row's blocks, one b x cols strip; with
-                // F.skip, only its runs of blocks the sweep did not read
-                const int64_t k0 = F.rows.row_ptr[pr], k1 = F.rows.row_ptr[pr + 1];
-                b = F.rows.row_b[pr];
-                base = reinterpret_cast<const unsigned char*>(F.val + (k1 > k0 ? F.rows.blk_voff[k0] : 0));
-                esz = sizeof(TA);
-                if (F.skip != nullptr) {
-                    const int kc = max(1, chunk_bytes / (b * esz));
-                    // the chunks of every run of streamed blocks: counted, then posted
-                    int nchunk = 0;
-                    for (int pass = 0; pass < 2; ++pass) {
-                        int col = 0, ch = 0;
-                        for (int64_t k = k0; k <= k1; ++k) {
-                            int run0 = col;
-                            while (k < k1 && !F.skip[k]) { col += F.rows.blk_nc[k]; ++k; }
-                            for (int c0 = run0; c0 < col; c0 += kc, ++ch) {
-                                if (pass == 0) continue;
-                                if (!mbar_wait(empty + stage, phase ^ 1u, S.spin_limit)) atomicExch(S.status, 1);
-                                StreamMeta m;
-                                m.task = (int)t; m.pr = pr; m.q = q; m.chunk = ch; m.nchunk = nchunk;
-                                m.skip = 0;
-                                m.col0 = c0;
-                                m.ncols = min(kc, col - c0);
-                                const uintptr_t src = reinterpret_cast<uintptr_t>(base + (size_t)c0 * b * esz);
-                                const uintptr_t a0 = src & ~(uintptr_t)15;
-                                const unsigned bytes = (unsigned)((size_t)m.ncols * b * esz);
-                                const unsigned len = (unsigned)(((src - a0) + bytes + 15) & ~(uintptr_t)15);
-                                m.shift = (int)((src - a0) / esz);
-                                meta[stage] = m;
-                                mbar_arrive_expect_tx(full + stage, len);
-                                bulk_copy_g2s(stages + (size_t)stage * stage_bytes, reinterpret_cast<const void*>(a0), len,
-                                              full + stage);
-                                if (++stage == nstage) { stage = 0; phase ^= 1u; }
-                            }
-                            if (k < k1) col += F.rows.blk_nc[k];      // a skipped block
-                        }
-                        nchunk = ch;
-                    }
-                    if (nchunk > 0) continue;
-                    cols = 0;                                        // nothing streamed: one empty chunk
-                } else {
-                    for (int64_t k = k0; k < k1; ++k) cols += F.rows.blk_nc[k];
-                }
-            } else if (q >= 0) {
-                if (FORWARD) { base = reinterpret_cast<const unsigned char*>(LD + R.lo_L[q]); cols = R.lo_nc[q]; esz = sizeof(TL); }
-                else { base = reinterpret_cast<const unsigned char*>(Aval + R.up_U[q]); cols = R.up_nc[q]; esz = sizeof(TU); }
-            } else if (q == -2) {
-                base = reinterpret_cast<const unsigned char*>(LD + R.dinv_off[pr]);
-                cols = b;
-                esz = sizeof(TL);
-            }
-            const int kc = cols > 0 ? max(1, min(cols, chunk_bytes / (b * esz))) : 1;
-            const int nchunk = cols > 0 ? (cols + kc - 1) / kc : 1;
-            for (int ch = 0; ch < nchunk; ++ch) {
-                if (!mbar_wait(empty + stage, phase ^ 1u, S.spin_limit)) atomicExch(S.status, 1);
-                StreamMeta m;
-                m.task = (int)t; m.pr = pr; m.q = q; m.chunk = ch; m.nchunk = nchunk;
-                m.skip = 0;
-                m.col0 = ch * kc;
-                m.ncols = cols > 0 ? min(kc, cols - ch * kc) : 0;
-                m.shift = 0;
-                if (cols > 0) {
-                    const uintptr_t src = reinterpret_cast<uintptr_t>(base + (size_t)m.col0 * b * esz);
-                    const uintptr_t a0 = src & ~(uintptr_t)15;
-                    const unsigned bytes = (unsigned)((size_t)m.ncols * b * esz);
+                if (ncols > 0) {
+                    const unsigned bytes = (unsigned)((size_t)ncols * b * esz);
                     const unsigned len = (unsigned)(((src - a0) + bytes + 15) & ~(uintptr_t)15);
-                    m.shift = (int)((src - a0) / esz);
-                    meta[stage] = m;
                     mbar_arrive_expect_tx(full + stage, len);
                     bulk_copy_g2s(stages + (size_t)stage * stage_bytes, reinterpret_cast<const void*>(a0), len, full + stage);
                 } else {
-                    meta[stage] = m;
                     mbar_arrive(full + stage);
                 }
+                ++ch;
                 if (++stage == nstage) { stage = 0; phase ^= 1u; }
+            };
+            // a strip of cols columns, staged from column col0 on; its last chunk carries `end`
+            auto post_strip = [&](const void* base, int col0, int cols, int esz, int end) {
+                const int kc = chunk_cols(cols, b, esz, chunk_bytes);
+                for (int c = 0; c < cols; c += kc)
+                    post(reinterpret_cast<const unsigned char*>(base) + (size_t)c * b * esz, col0 + c, min(kc, cols - c), esz,
+                         c + kc >= cols ? end : 0, 0);
+            };
+            auto chunks = [&](int cols, int esz) {
+                const int kc = chunk_cols(cols, b, esz, chunk_bytes);
+                return (cols + kc - 1) / kc;
+            };
+            if (row_frozen(mask, d.row)) {
+                // a frozen system's row: one empty chunk, nothing read or written
+                nchunk = 1;
+                post(nullptr, 0, 0, 1, 0, 1);
+            } else if (MV && d.code == SW_MATVEC) {
+                // the row's blocks, with F.skip only those the sweep did not read
+                const int64_t k0 = F.rows.row_ptr[d.row], k1 = F.rows.row_ptr[d.row + 1];
+                for (int64_t k = k0; k < k1; ++k)
+                    if (F.skip == nullptr || !F.skip[k]) nchunk += chunks(F.rows.blk_nc[k], sizeof(TA));
+                int col = 0;
+                for (int64_t k = k0; k < k1; ++k) {
+                    const int nc = F.rows.blk_nc[k];
+                    if (F.skip == nullptr || !F.skip[k]) post_strip(F.val + F.rows.blk_voff[k], col, nc, sizeof(TA), 0);
+                    col += nc;
+                }
+                if (nchunk == 0) { nchunk = 1; post(nullptr, 0, 0, 1, 0, 0); }   // nothing streamed
+            } else if (d.code == SW_ROW) {
+                if (FORWARD) {
+                    // the row's L blocks follow one another in LD
+                    nchunk = max(1, chunks(d.cols, sizeof(TL)));
+                    if (d.cols == 0) post(nullptr, 0, 0, 1, 0, 0);
+                    else post_strip(LD + d.off, 0, d.cols, sizeof(TL), 0);
+                } else {
+                    for (int e = d.q0; e < d.q1; ++e) nchunk += chunks(R.up_nc[e], sizeof(TU));
+                    nchunk += chunks(b, sizeof(TL));
+                    int col = 0;
+                    for (int e = d.q0; e < d.q1; ++e) {
+                        post_strip(Aval + R.up_U[e], col, R.up_nc[e], sizeof(TU), e == d.q1 - 1);
+                        col += R.up_nc[e];
+                    }
+                    post_strip(LD + d.off, 0, b, sizeof(TL), 0);
+                }
+            } else {
+                const int esz = (FORWARD || d.code == SW_DIAG) ? (int)sizeof(TL) : (int)sizeof(TU);
+                // slices s0 .. s0 + nsl - 1 of the cut of nc columns, side by side
+                const int ns = sweep_slices(b);
+                auto cut = [&](int s) { return d.nc * (d.s0 + s) / ns - d.nc * d.s0 / ns; };
+                for (int s = 0; s < d.nsl; ++s) nchunk += max(1, chunks(cut(s + 1) - cut(s), esz));
+                for (int s = 0; s < d.nsl; ++s) {
+                    const int c0 = cut(s), cols = cut(s + 1) - c0;
+                    const int64_t o = d.off + (int64_t)c0 * b;
+                    if (cols == 0) post(nullptr, 0, 0, 1, 1, 0);
+                    else if (FORWARD || d.code == SW_DIAG) post_strip(LD + o, c0, cols, esz, 1);
+                    else post_strip(Aval + o, c0, cols, esz, 1);
+                }
             }
+            if (++slot == SS_SLOTS) slot = 0;
+            t = tn;
+            if (t < (unsigned)ntasks) slots[slot] = T.task[t];
         }
+        if (!mbar_wait(empty + stage, phase ^ 1u, S.spin_limit)) atomicExch(S.status, 1);
+        meta[stage].task = -1;
+        mbar_arrive(full + stage);
+        return;
     }
 
     // ---------------------------------------------------------------- consumers
     const int ctid = tid;
     int stage = 0;
     unsigned phase = 0;
-    int pr = 0, q = 0, b = 0, G = 1, r = 0, g = 0;
+    int slot = 0, b = 0, G = 1, r = 0, g = 0;
+    int sl = 0;                                  // slice of the task being summed; SW_ROW: 1 once U is done
+    TX own = TX(0);                              // SW_ROW: the row's v (forward) or z (backward), fetched before the wait
     ACC acc[RPT];
     for (;;) {
         if (!mbar_wait(full + stage, phase, S.spin_limit)) { if (ctid == 0) atomicExch(S.status, 1); }
@@ -387,62 +477,120 @@ __global__ void __launch_bounds__(32 * CW + 32)
             if (++stage == nstage) { stage = 0; phase ^= 1u; }
             continue;
         }
+        slot = m.task;
+        const StreamTask& d = slots[slot];
+        const int code = d.code;
         if (m.chunk == 0) {
-            pr = m.pr;
-            q = m.q;
-            b = (MV && q == -3) ? F.rows.row_b[pr] : R.prow_b[pr];
+            b = d.b;
+            sl = 0;
             if (b <= NC) { G = NC / b; r = ctid % b; g = ctid / b; }
             else { G = 1; r = ctid; g = 0; }
             #pragma unroll
             for (int rr = 0; rr < RPT; ++rr) acc[rr] = 0;
-            if (MV && q == -3) {
+            if (MV && code == SW_MATVEC) {
                 // every column segment of the row published by the sweep, then staged
-                const int64_t k0 = F.rows.row_ptr[pr], k1 = F.rows.row_ptr[pr + 1];
-                if (ctid == 0)
-                    for (int64_t k = k0; k < k1; ++k)
+                // (the blocks' offsets fetched before the wait)
+                const int64_t k0 = F.rows.row_ptr[d.row], k1 = F.rows.row_ptr[d.row + 1];
+                const int nb = (int)(k1 - k0);
+                if (nb <= SS_BLKS) {
+                    if (ctid < nb) {
+                        s_nc[ctid] = F.rows.blk_nc[k0 + ctid];
+                        s_x[ctid] = (F.skip == nullptr || !F.skip[k0 + ctid]) ? F.rows.blk_xoff[k0 + ctid] : -1;
+                    }
+                    if (ctid < nb && !wait_flag(S.flags, F.col_prow[k0 + ctid], S.epoch, S.spin_limit)) atomicExch(S.status, 1);
+                    consumers_sync<NC>();
+                    // the segments side by side; four loads of a thread go out together
+                    int total = 0;
+                    for (int k = 0; k < nb; ++k) total += s_nc[k];
+                    for (int c0 = ctid; c0 < total; c0 += 4 * NC) {
+                        TX val4[4];
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            int c = c0 + u * NC, k = 0;
+                            while (k < nb && c >= s_nc[k]) c -= s_nc[k++];
+                            val4[u] = (k < nb && s_x[k] >= 0) ? ld_cg(zx + s_x[k] + c) : TX(0);
+                        }
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (c0 + u * NC < total) xs[c0 + u * NC] = cvt<ACC>(val4[u]);
+                    }
+                } else {
+                    for (int64_t k = k0 + ctid; k < k1; k += NC)
                         if (!wait_flag(S.flags, F.col_prow[k], S.epoch, S.spin_limit)) atomicExch(S.status, 1);
-                consumers_sync<NC>();
+                    consumers_sync<NC>();
+                    int off = 0;
+                    for (int64_t k = k0; k < k1; ++k) {
+                        const int nc = F.rows.blk_nc[k];
+                        if (F.skip == nullptr || !F.skip[k]) {
+                            const TX* xp = zx + F.rows.blk_xoff[k];
+                            for (int c = ctid; c < nc; c += NC) xs[off + c] = cvt<ACC>(ld_cg(xp + c));
+                        }
+                        off += nc;
+                    }
+                }
+            } else if (code == SW_ROW) {
+                // thread c stages column c of the entries' columns side by side
+                // (and c + NC): its address before the wait
+                const int32_t* par = FORWARD ? R.lo_par : R.up_par;
+                const int32_t* ncs = FORWARD ? R.lo_nc : R.up_nc;
+                constexpr int CPT = (SW_ROW_COLS + NC - 1) / NC;
+                const TX* at[CPT];
+                #pragma unroll
+                for (int u = 0; u < CPT; ++u) at[u] = nullptr;
                 int off = 0;
-                for (int64_t k = k0; k < k1; ++k) {
-                    const int nc = F.rows.blk_nc[k];
-                    if (F.skip == nullptr || !F.skip[k]) {
-                        const TX* xp = zx + F.rows.blk_xoff[k];
-                        for (int c = ctid; c < nc; c += NC) xs[off + c] = cvt<ACC>(ld_cg(xp + c));
+                for (int e = d.q0; e < d.q1; ++e) {
+                    const int nc = ncs[e];
+                    const TX* zp = zx + R.z_off[par[e]];
+                    #pragma unroll
+                    for (int u = 0; u < CPT; ++u) {
+                        const int c = ctid + u * NC - off;
+                        if (c >= 0 && c < nc) at[u] = zp + c;
                     }
                     off += nc;
                 }
+                if (ctid < b) own = (FORWARD || d.src == 1) ? v[d.vrow + ctid] : zx[d.zrow + ctid];
+                for (int e = d.q0 + ctid; e < d.q1; e += NC)
+                    if (!wait_flag(S.flags, par[e], S.epoch, S.spin_limit)) atomicExch(S.status, 1);
                 consumers_sync<NC>();
-            } else if (q >= 0) {
-                const int par = FORWARD ? R.lo_par[q] : R.up_par[q];
-                const int nc = FORWARD ? R.lo_nc[q] : R.up_nc[q];
-                if (ctid == 0 && !wait_flag(S.flags, par, S.epoch, S.spin_limit)) atomicExch(S.status, 1);
-                consumers_sync<NC>();
-                const TX* zp = zx + R.z_off[par];
-                for (int c = ctid; c < nc; c += NC) xs[c] = cvt<ACC>(ld_cg(zp + c));
-                consumers_sync<NC>();
-            } else if (q == -2) {
-                // t_r = z_r - sum of the row's U partials, in entry order
-                const int q0 = R.up_ptr[pr], q1 = R.up_ptr[pr + 1];
-                if (q1 > q0 && ctid == 0 && !wait_flag(T.ready, pr, S.epoch, S.spin_limit)) atomicExch(S.status, 1);
-                consumers_sync<NC>();
-                for (int i = ctid; i < b; i += NC) {
-                    ACC s = 0;
-                    for (int qq = q0; qq < q1; ++qq) s += ld_cg(part + T.part_off[qq] + i);
-                    xs[i] = cvt<ACC>(from_d<TX>(to_d(ld_cg(zx + R.z_off[pr] + i)) - (double)s));
+                #pragma unroll
+                for (int u = 0; u < CPT; ++u)
+                    if (at[u] != nullptr) xs[ctid + u * NC] = cvt<ACC>(ld_cg(at[u]));
+                if (!FORWARD && d.q1 == d.q0 && ctid < b) xs[ctid] = cvt<ACC>(own);      // inv(D) alone
+            } else {
+                // slice of an entry or of inv(D): see StreamTask
+                const int wt = d.wait;
+                if (ctid == 0 && wt >= 0) {
+                    const unsigned* p = (FORWARD ? T.count : code == SW_DIAG ? T.count : T.dcount) + d.par;
+                    if (!(wt == 0 ? wait_flag(S.flags, d.par, S.epoch, S.spin_limit) : wait_count(p, (unsigned)wt, S.spin_limit)))
+                        atomicExch(S.status, 1);
                 }
                 consumers_sync<NC>();
-            } else {
-                // forward row without lower entries: z_r = v_r
-                for (int i = ctid; i < b; i += NC) zx[R.z_off[pr] + i] = v[R.v_off[pr] + i];
-                consumers_sync<NC>();
-                if (ctid == 0) st_release(S.flags + pr, S.epoch);
+                const TX* base = (d.src == 1 ? v : zx) + d.seg;
+                const ACC* pp = part + d.pseg;
+                for (int c = ctid; c < d.cols; c += NC) {
+                    const double x0 = d.src == 2 ? 0.0 : to_d(ld_cg(base + c));
+                    const ACC s = sum_partials_at(pp + c, d.npart, d.pb, ACC(0));
+                    xs[c] = cvt<ACC>(from_d<TX>(d.src == 2 ? (double)s : x0 - (double)s));
+                }
             }
+            consumers_sync<NC>();
+        }
+        if (!FORWARD && code == SW_ROW && sl == 1) {
+            // the row's U products are complete: t_r = z_r - sum takes the segments' place
+            stream_reduce<NC, RPT>(red, b, r, g, G, ctid, acc);
+            if (ctid < b) {
+                part[d.out + ctid] = acc[0];                // read by the row's matvec task
+                xs[ctid] = cvt<ACC>(from_d<TX>(to_d(own) - (double)acc[0]));
+            }
+            acc[0] = 0;
+            sl = 2;
+            consumers_sync<NC>();
         }
         if (m.ncols > 0) {
             const unsigned char* sb = stages + (size_t)stage * stage_bytes;
-            if (MV && q == -3)
+            if (MV && code == SW_MATVEC)
                 stream_chunk<NC, RPT, TA, ACC>(reinterpret_cast<const TA*>(sb) + m.shift, xs + m.col0, b, m.ncols, r, g, G, acc);
-            else if (FORWARD || q == -2)
+            else if (FORWARD || code == SW_DIAG || (code == SW_ROW && (sl == 2 || d.q1 == d.q0)))
                 stream_chunk<NC, RPT, TL, ACC>(reinterpret_cast<const TL*>(sb) + m.shift, xs + m.col0, b, m.ncols, r, g, G, acc);
             else
                 stream_chunk<NC, RPT, TU, ACC>(reinterpret_cast<const TU*>(sb) + m.shift, xs + m.col0, b, m.ncols, r, g, G, acc);
@@ -450,25 +598,34 @@ __global__ void __launch_bounds__(32 * CW + 32)
         __syncwarp();
         if (lane == 0) mbar_arrive(empty + stage);
         if (++stage == nstage) { stage = 0; phase ^= 1u; }
-        if (m.chunk != m.nchunk - 1 || q == -1) continue;
+        if (m.chunk != m.nchunk - 1) {
+            if (!m.end) continue;
+            if (code == SW_ROW) { sl = 1; continue; }
+            // a slice with others after it in the task: its partial sums
+            stream_reduce<NC, RPT>(red, b, r, g, G, ctid, acc);
+            ACC* o = part + d.out + (int64_t)sl * b;
+            #pragma unroll
+            for (int rr = 0; rr < RPT; ++rr) {
+                const int i = (b <= NC) ? (rr == 0 ? ctid : b) : ctid + NC * rr;
+                if (i < b) o[i] = acc[rr];
+                acc[rr] = 0;
+            }
+            ++sl;
+            consumers_sync<NC>();        // the row sums' scratch is written again
+            continue;
+        }
 
         // ------------------------------------------------ the task's last chunk
         stream_reduce<NC, RPT>(red, b, r, g, G, ctid, acc);
-        if (MV && q == -3) {
-            // y_r = A_r z and its sum of squares, as the streamed matvec writes
-            // them (with F.skip: plus the row's U partials, in entry order)
+        if (MV && code == SW_MATVEC) {
+            // y_r = A_r z and its sum of squares (with F.skip: plus the row's U partials, in order)
             double sq = 0.0;
-            const int64_t yo = F.rows.row_yoff[pr];
-            const int u0 = F.skip != nullptr ? R.up_ptr[pr] : 0, u1 = F.skip != nullptr ? R.up_ptr[pr + 1] : 0;
+            const int64_t yo = F.rows.row_yoff[d.row];
             #pragma unroll
             for (int rr = 0; rr < RPT; ++rr) {
                 const int i = (b <= NC) ? (rr == 0 ? ctid : b) : ctid + NC * rr;
                 if (i < b) {
-                    if (u1 > u0) {
-                        ACC s = 0;
-                        for (int u = u0; u < u1; ++u) s += ld_cg(part + T.part_off[u] + i);
-                        acc[rr] += s;
-                    }
+                    if (F.skip != nullptr) acc[rr] += sum_partials_at(part + d.rbase + i, d.nall, b, ACC(0));
                     const TX o = from_d<TX>((double)acc[rr]);
                     F.y[yo + i] = o;
                     const double od = to_d(o);
@@ -477,49 +634,49 @@ __global__ void __launch_bounds__(32 * CW + 32)
             }
             if (F.row_sumsq != nullptr) {
                 const double s2 = consumers_sum<NC>(sq, scratch, ctid);
-                if (ctid == 0) F.row_sumsq[pr] = s2;
+                if (ctid == 0) F.row_sumsq[d.row] = s2;
             }
             consumers_sync<NC>();        // xs, red and scratch are reused by the next task
             continue;
         }
-        if (q == -2) {
-            // x_r = inv(D_r) t_r: the row is complete
-            if (b <= NC) { if (ctid < b) zx[R.z_off[pr] + ctid] = from_d<TX>((double)acc[0]); }
+        if (code == SW_ROW) {
+            // the row is complete: z_r = v_r - sum, or inv(D_r) t_r
+            if (ctid < b) {
+                const double x = FORWARD ? to_d(own) - (double)acc[0] : (double)acc[0];
+                zx[d.zrow + ctid] = from_d<TX>(x);
+            }
+            consumers_sync<NC>();
+            if (ctid == 0) st_release(S.flags + d.row, S.epoch);
+            continue;
+        }
+        // the slice's partial sums, counted; the last forward slice, or slice of
+        // inv(D), of the row writes z_r
+        const bool none = FORWARD && d.q1 == d.q0;         // a row without entries: z_r = v_r
+        if (none) {}
+        else {
+            ACC* o = part + d.out + (int64_t)sl * b;
+            if (b <= NC) { if (ctid < b) o[ctid] = acc[0]; }
             else {
                 #pragma unroll
                 for (int rr = 0; rr < RPT; ++rr)
-                    if (ctid + NC * rr < b) zx[R.z_off[pr] + ctid + NC * rr] = from_d<TX>((double)acc[rr]);
+                    if (ctid + NC * rr < b) o[ctid + NC * rr] = acc[rr];
             }
-            consumers_sync<NC>();
-            if (ctid == 0) st_release(S.flags + pr, S.epoch);
+        }
+        consumers_sync<NC>();
+        if (!FORWARD && code == SW_ENTRY) {
+            if (ctid == 0) red_release(T.count + d.row, (unsigned)d.nsl);
             continue;
         }
-        if (b <= NC) { if (ctid < b) part[T.part_off[q] + ctid] = acc[0]; }
-        else {
-            #pragma unroll
-            for (int rr = 0; rr < RPT; ++rr)
-                if (ctid + NC * rr < b) part[T.part_off[q] + ctid + NC * rr] = acc[rr];
+        if (ctid == 0)
+            s_last = atom_add_acq_rel((FORWARD ? T.count : T.dcount) + d.row, (unsigned)d.nsl) + (unsigned)d.nsl == (unsigned)d.nall;
+        consumers_sync<NC>();
+        if (!s_last) continue;
+        for (int i = ctid; i < b; i += NC) {
+            const ACC s = sum_partials_at(part + d.rbase + i, none ? 0 : d.nall, b, ACC(0));
+            zx[d.zrow + i] = from_d<TX>(FORWARD ? to_d(v[d.vrow + i]) - (double)s : (double)s);
         }
         consumers_sync<NC>();
-        const int q0 = FORWARD ? R.lo_ptr[pr] : R.up_ptr[pr];
-        const int q1 = FORWARD ? R.lo_ptr[pr + 1] : R.up_ptr[pr + 1];
-        if (ctid == 0) {
-            const unsigned old = atom_add_acq_rel(T.row_count + pr, 1u);
-            const bool last = ((old + 1u) % (unsigned)(q1 - q0)) == 0u;
-            if (last && !FORWARD) st_release(T.ready + pr, S.epoch);
-            s_last = last;
-        }
-        consumers_sync<NC>();
-        if constexpr (FORWARD) {
-            if (!s_last) continue;
-            for (int i = ctid; i < b; i += NC) {
-                ACC s = 0;
-                for (int qq = q0; qq < q1; ++qq) s += ld_cg(part + T.part_off[qq] + i);
-                zx[R.z_off[pr] + i] = from_d<TX>(to_d(v[R.v_off[pr] + i]) - (double)s);
-            }
-            consumers_sync<NC>();
-            if (ctid == 0) st_release(S.flags + pr, S.epoch);
-        }
+        if (ctid == 0) st_release(S.flags + d.row, S.epoch);
     }
 }
 
