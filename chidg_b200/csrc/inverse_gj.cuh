@@ -35,10 +35,13 @@
 //
 // Bound by that chain (654 cycles a pivot step at 40 rows, 1035 at 135: the
 // latencies of a barrier, a reduction over the warp and eight dependent
-// multiply-adds), not by the FP64 rate or by memory.  A launch of up to 148
-// blocks takes 26 us at 40 rows (54 with one step per barrier pair over the
-// whole block), 100 us at 135 rows (142), 285 us at 320 rows for up to 29
-// blocks, the clusters of five that fit the chip, and 1.37 ms for 120.  The
+// multiply-adds), not by the FP64 rate or by memory; the pivots' divisions run
+// beside the warps' search and cost nothing measurable against a seed and a
+// correction step (28.0, 96.4 and 279 us a launch of 40, 135 and 320 rows; 28.8,
+// 97.2 and 283).  A launch of up to 148 blocks takes 28 us at 40 rows (54 with one
+// step per barrier pair over the whole block), 96 us at 135 rows (142), 279 us at
+// 320 rows for as many blocks as clusters of five fit the chip (24 to 29), and
+// 1.37 ms for 120.  The
 // form with the rows of a 320-row block in global memory took 1.26 ms for any
 // number up to 148, so a level of 110 to 148 such blocks alone is up to a
 // third slower here; the levels of a mesh grow from one block and shrink again,
@@ -125,19 +128,6 @@ __device__ __forceinline__ void gj_wait(uint64_t* bar, unsigned parity, long lon
         if (ok) return;
         if (clock64() - t0 > limit) { limit = 0; return; }
     }
-}
-
-// 1 / x for the elimination: a 20-bit seed and one step of third order,
-// y (1 + e + e^2) with e = 1 - x y (error e^3, below rounding): three dependent
-// operations in the chain of the pivot steps.  Magnitudes whose seed would be
-// flushed or overflow, zeros, infinities and NaN take the division.
-__device__ __forceinline__ double gj_reciprocal(double x) {
-    const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-    if (ex - 64u > 1918u) return 1.0 / x;         // |x| outside 2^-959 .. 2^960
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
 }
 
 // two doubles to shared memory where p is set, without a branch
@@ -300,7 +290,11 @@ __device__ __forceinline__ void gj_block(unsigned char* gj_raw, double* D, int b
                 // (checked beside that) do the low words decide
                 const unsigned hi = (mine && !used) ? (unsigned)__double2hiint(r[0]) | 0x80000000u : 0u;
                 const unsigned lo = (unsigned)__double2loint(r[0]);
-                const double rcp = gj_reciprocal(hi != 0u ? r[0] : 1.0);
+                // (opaque, or the compiler divides by a padding row's zero after all: the
+                // division's slow path, 5 to 10 % of a step)
+                double div = hi != 0u ? r[0] : 1.0;
+                asm("" : "+d"(div));
+                const double rcp = 1.0 / div;
                 const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
                 const bool top = hi == mhi && hi != 0u;
                 auto propose = [&](bool mine_) {

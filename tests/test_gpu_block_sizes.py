@@ -50,3 +50,28 @@ def test_factors_and_sweeps_by_block_size(nvars, nterms):
         if np.any(o):
             assert _relerr(LDg[voff[k]:voff[k] + b * b], o) < tol
     assert _relerr(Mg.apply(Ag, api.ChidgVector(Ag, v)).download(), Mo.apply(v)) < tol
+
+
+@pytest.mark.parametrize("nvars,nterms", [(1, 1), (5, 8), (5, 27), (5, 64), (6, 64)], ids=["b1", "b40", "b135", "b320", "b384"])
+def test_inverse_of_a_diagonal_block_is_the_correctly_rounded_quotient(nvars, nterms):
+    """Pivots divide: a diagonal block's inverse holds 1 / d, bit for bit, over
+    mantissas and the exponents of normal quotients and beyond (2^-1022 .. 2^1023)."""
+    b = nvars * nterms
+    pat = mesh.box_pattern(1 << 18 if b == 1 else 4, 1, 1, nvars, nterms)
+    voff, nval = pat.value_offsets()
+    diag = voff[np.asarray(pat.blk_face) == mesh.DIAG]
+    rng = np.random.default_rng(64)
+    d = np.ldexp(rng.uniform(1.0, 2.0, diag.size * b) * rng.choice([-1.0, 1.0], diag.size * b),
+                 np.where(np.arange(diag.size * b) % 2, rng.integers(-1022, 1023, diag.size * b), 0))
+    d = d.reshape(diag.size, b)
+    vals = np.zeros(nval)
+    at = diag[:, None] + (b + 1) * np.arange(b)
+    vals[at] = d
+    A = api.ChidgMatrix(pat)
+    A.upload(vals)
+    M = api.create_preconditioner("jacobi")
+    M.update(A)
+    want = np.zeros(nval)
+    want[at] = 1.0 / d
+    inside = (diag[:, None] + np.arange(b * b)).ravel()
+    assert np.array_equal(M.LD()[inside], want[inside])
