@@ -3,6 +3,7 @@
 // programme builders that turn the reference's block-ILU0 / RAS+ILU0 loops into
 // level-scheduled GPU sweeps.  The FGMRES driver lives in fgmres.cu.
 #include "chidg_gpu_internal.cuh"
+#include "inverse_rows.cuh"
 
 #include <tuple>
 #include <type_traits>
@@ -1753,6 +1754,30 @@ extern "C" int chidg_gpu_precon_stamp(chidg_gpu_precon* M, int64_t* s) {
     return CHIDG_GPU_OK;
 }
 
+// Whether `count` blocks of up to bmax rows are inverted sooner by one CTA a
+// block (k_block_inverse_rows, one CTA an SM) than by clusters of C CTAs
+// (k_block_inverse_gj).  Alone a block takes 2.6 (216 rows) to 3.7 times (352) as
+// long in the first form, but 148 blocks run at a time in it, and some 50, 35 or
+// 26 clusters of three, four or five.  bmax / 75 lies between the ratios measured
+// at 216 to 352 rows and 30 to 740 blocks; where it chooses the first form that
+// was never slower by more than 2 %, and the other choice cost up to 10 % at two
+// waves of it.  ms of an update of one level, clusters / one CTA a block: 240 rows,
+// 100 blocks 0.60 / 0.61, 148 0.80 / 0.65, 740 3.30 / 3.02; 270 rows, 60 blocks
+// 0.49 / 0.76, 100 0.95 / 0.78, 740 5.38 / 3.89; 320 rows, 100 blocks 1.18 / 1.10,
+// 148 1.75 / 1.21, 200 2.32 / 2.23, 740 8.30 / 5.90.  Up to 208 rows clusters of
+// two always win (148 blocks 0.38 / 0.50).
+template <typename K>
+static bool rows_inverse_wins(chidg_gpu_ctx* ctx, K kern, const cudaLaunchConfig_t& cfg, int C, int count, int bmax) {
+    if (bmax <= 208 || bmax > RP_MAX) return false;
+    int& slots = ctx->gj_slots[C];
+    if (slots == 0 && (cudaOccupancyMaxActiveClusters(&slots, kern, &cfg) != cudaSuccess || slots < 1)) {
+        cudaGetLastError();
+        slots = 1;
+    }
+    const long long waves = (count + slots - 1) / slots, rows_waves = (count + ctx->nsm - 1) / ctx->nsm;
+    return 75 * waves > bmax * rows_waves;
+}
+
 // the inverses of rows row_begin .. + count of the factorisation order, blocks of at most bmax rows
 static int launch_inverse(chidg_gpu_precon* M, int row_begin, int count, int bmax) {
     chidg_gpu_ctx* ctx = M->ctx;
@@ -1768,20 +1793,21 @@ static int launch_inverse(chidg_gpu_precon* M, int row_begin, int count, int bma
         // products take about as long as the panel with two tiles a warp
         const int threads = 32 * std::min(GJ_THREADS / 32, T + (bmax <= 64 ? 2 : 7));
         const size_t smem = gj_smem(bmax, C);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(count * C));
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = ctx->stream;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)C;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = C > 1 ? 1 : 0;
         auto go = [&](auto kern) -> int {
             const int s2 = raise_smem_limit((const void*)kern, smem);
             if (s2) return fail(ctx, s2, "block inverse shared memory");
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3((unsigned)(count * C));
-            cfg.blockDim = dim3((unsigned)threads);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = ctx->stream;
-            cudaLaunchAttribute at{};
-            at.id = cudaLaunchAttributeClusterDimension;
-            at.val.clusterDim.x = (unsigned)C;
-            at.val.clusterDim.y = at.val.clusterDim.z = 1;
-            cfg.attrs = &at;
-            cfg.numAttrs = C > 1 ? 1 : 0;
+            if (rows_inverse_wins(ctx, kern, cfg, C, count, bmax)) return 1;
             const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, LD, off, pb, pe, rows, row_begin, ctx->d_status, C, T);
             if (e != cudaSuccess) {
                 cudaGetLastError();
@@ -1790,7 +1816,13 @@ static int launch_inverse(chidg_gpu_precon* M, int row_begin, int count, int bma
             return check_launch(ctx, "k_block_inverse_gj");
         };
         if (C == 1) return T <= 4 ? go(k_block_inverse_gj<false, 4>) : go(k_block_inverse_gj<false, 8>);
-        return T <= 8 ? go(k_block_inverse_gj<true, 8>) : go(k_block_inverse_gj<true, 12>);
+        st = T <= 8 ? go(k_block_inverse_gj<true, 8>) : go(k_block_inverse_gj<true, 12>);
+        if (st != 1) return st;
+        const size_t rsmem = rp_smem_bytes(bmax);
+        if ((st = raise_smem_limit((const void*)k_block_inverse_rows, rsmem)))
+            return fail(ctx, st, "row inverse shared memory");
+        k_block_inverse_rows<<<count, RP_THREADS, rsmem, ctx->stream>>>(LD, off, pb, pe, rows, row_begin, ctx->d_status, bmax);
+        return check_launch(ctx, "k_block_inverse_rows");
     }
     // larger blocks: panels of 16 columns (8 above 704 rows) in shared memory,
     // (2 NB + 1) b doubles

@@ -147,6 +147,7 @@ struct chidg_gpu_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int nsm = 148;
+    int gj_slots[9] = {};            // clusters of that many CTAs the inverses hold at a time (0: not asked yet)
     std::string err;
     int32_t err_elem = -1;
     int64_t launches = 0;

@@ -40,12 +40,10 @@
 // correction step (28.0, 96.4 and 279 us a launch of 40, 135 and 320 rows; 28.8,
 // 97.2 and 283).  A launch of up to 148 blocks takes 28 us at 40 rows (54 with one
 // step per barrier pair over the whole block), 96 us at 135 rows (142), 279 us at
-// 320 rows for as many blocks as clusters of five fit the chip (24 to 29), and
-// 1.37 ms for 120.  The
-// form with the rows of a 320-row block in global memory took 1.26 ms for any
-// number up to 148, so a level of 110 to 148 such blocks alone is up to a
-// third slower here; the levels of a mesh grow from one block and shrink again,
-// and all of them together take 12.0 ms, before 31.4 (9 x 8 x 10 elements).
+// 320 rows for as many blocks as clusters of five fit the chip (24 to 29).  Levels
+// of many more blocks above 208 rows are inverted by inverse_rows.cuh, one CTA a
+// block.  All levels of 9 x 8 x 10 elements of order 3 take 12.0 ms, 31.4 in that
+// form alone.
 //
 // After the last panel the stored matrix S satisfies S(p_k, j) =
 // inv(A)(k, p_j); the write-back undoes the permutation.  A zero pivot records

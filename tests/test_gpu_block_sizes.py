@@ -6,7 +6,7 @@ one-task rows (up to 64) and column slices (three up to 160, eight above)."""
 import numpy as np
 import pytest
 
-from chidg_b200 import api, mesh
+from chidg_b200 import _lib, api, mesh
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -75,3 +75,38 @@ def test_inverse_of_a_diagonal_block_is_the_correctly_rounded_quotient(nvars, nt
     want[at] = 1.0 / d
     inside = (diag[:, None] + np.arange(b * b)).ravel()
     assert np.array_equal(M.LD()[inside], want[inside])
+
+
+@pytest.mark.parametrize("sizes", [(216,), (257,), (320,), (352,), (209, 224, 243, 320), (321, 337, 352)],
+                         ids=lambda s: "-".join(map(str, s)))
+def test_inverses_of_many_large_blocks(sizes):
+    """More blocks of 209 to 352 rows in one level than clusters fit the chip:
+    one CTA a block.  Every second block's rows are shuffled; a singular one is
+    reported by its element."""
+    rng = np.random.default_rng(65)
+    pat = mesh.box_pattern(120, 1, 1, 1, sizes[0])
+    pat.elem_nterms[:] = rng.choice(sizes, pat.nelem)
+    voff, nval = pat.value_offsets()
+    diag = voff[np.asarray(pat.blk_face) == mesh.DIAG]
+    vals = np.zeros(nval)
+    blocks = []
+    for k, (o, b) in enumerate(zip(diag, pat.elem_nterms)):
+        D = np.eye(b) + 0.6 / np.sqrt(b) * rng.uniform(-1.0, 1.0, (b, b))
+        blocks.append(D[rng.permutation(b)] if k % 2 else D)
+        vals[o:o + b * b] = blocks[-1].ravel(order="F")
+    A = api.ChidgMatrix(pat)
+    A.upload(vals)
+    M = api.create_preconditioner("jacobi")
+    M.update(A)
+    LD = M.LD()
+    for o, D in zip(diag, blocks):
+        b = len(D)
+        # backward error of an inverse from LU with partial pivoting, times the condition
+        tol = 64 * b * np.finfo(float).eps * np.linalg.cond(D)
+        assert _relerr(LD[o:o + b * b].reshape(b, b).T, np.linalg.inv(D)) < tol
+    b = int(pat.elem_nterms[77])
+    vals[diag[77]:diag[77] + b * b].reshape(b, b)[:, 5] = 0.0              # a zero row
+    A.upload(vals)
+    with pytest.raises(_lib.ChidgGpuError) as ei:
+        M.update(A)
+    assert ei.value.code == _lib.ESINGULAR and ei.value.element == 77
