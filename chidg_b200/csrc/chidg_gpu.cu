@@ -1023,6 +1023,7 @@ int find_trans(const chidg_gpu_matrix* A, int p, int t, int e) {
 // ILU0 / Jacobi on a single rank: one programme row per matrix row.
 static int build_ilu0(const chidg_gpu_matrix* A, bool jacobi, IluProgram& P, std::string& err) {
     P = IluProgram();
+    P.diagonal = jacobi;
     P.n_ext = A->n;
     P.nlocal_rows = A->nrow;
     // programme row id == matrix row id (e*ntime+t)
@@ -1076,6 +1077,7 @@ static int build_hb(const chidg_gpu_matrix* A, IluProgram& P, std::string& err) 
     P.n_ext = A->n;
     P.nlocal_rows = A->nelem;
     P.assembled = true;
+    P.diagonal = true;
     P.asm_ptr.assign(1, 0);
     for (int e = 0; e < A->nelem; ++e) {
         const int b = A->bsize(e), B = b * A->ntime;
@@ -1286,7 +1288,7 @@ static void stream_layout(IluProgram& P) {
         int64_t size = 0;
         for (int pr = 0; pr < np; ++pr) {
             const auto& ents = (fwd ? P.lo : P.up)[pr];
-            const int b = P.prow_b[pr], ns = sweep_slices(b);
+            const int b = P.prow_b[pr], ns = P.slices(b);
             int cols = 0;
             for (const auto& en : ents) cols += en.nc;
             base[pr] = size;
@@ -1362,7 +1364,7 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
     for (int pr = 0; pr < np; ++pr) first[pr + 1] = first[pr] + (int)(fwd ? P.lo : P.up)[pr].size();
     for (int32_t pr : fwd ? P.fwd_rows : P.bwd_rows) {
         const auto& ents = (fwd ? P.lo : P.up)[pr];
-        const int b = P.prow_b[pr], ns = sweep_slices(b), ne = (int)ents.size();
+        const int b = P.prow_b[pr], ns = P.slices(b), ne = (int)ents.size();
         StreamTask t{};
         t.row = pr;
         t.b = b;
@@ -1373,6 +1375,7 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
         t.wait = -1;
         t.par = pr;
         t.pb = b;
+        t.ns = ns;
         if (whole[pr]) {
             t.code = SW_ROW;
             for (const auto& en : ents) t.cols += en.nc;
@@ -1383,7 +1386,7 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
             keyed.add(scale * (2 * lev[pr] - 1), t);
             continue;
         }
-        const int dstep = dlev[lev[pr]] >= many ? ns : 1;
+        const int dstep = dlev[lev[pr]] >= many && sweep_groups_slices(b, P.diagonal) ? ns : 1;
         if (!fwd)
             for (int s = 0; s < ns; s += dstep) {
                 StreamTask u = t;
@@ -1413,7 +1416,7 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
                 u.s0 = s;
                 u.nsl = step;
                 const int q = ents[e].parent, nc = ents[e].nc, c0 = nc * s / ns, nq = (int)(fwd ? P.lo : P.up)[q].size();
-                const int nsq = sweep_slices(nc);
+                const int nsq = P.slices(nc);
                 u.code = SW_ENTRY;
                 u.cols = nc * (s + step) / ns - c0;
                 u.off = (fwd ? ents[e].l_off : ents[e].a_off) + (int64_t)c0 * b;
@@ -2188,6 +2191,11 @@ static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV*
 // with matvec rows within FP64 solves, us, 24 / 26 KB: 24^3 of order 2 1137 / 1207
 // and 3229 / 2957, 12^3 250 / 240 and 555 / 496, 9 x 8 x 10 of order 3 346 / 362
 // and 882 / 851; 20 KB 1160, 249, 357 and 2941, 527, 950.
+// Programmes without couplings (Jacobi, precon_HB) have no chain, only as many
+// copies in flight as CTAs fit: their backward sweep takes two stages of 24 KB, four
+// CTAs an SM, and with the matvec rows of blocks up to 64 rows 20 KB (24^3 elements
+// of 40 rows, Jacobi: apply 125 us with the other defaults, 83 with these, with
+// matvec rows 614 and 397; 990 blocks of 280 rows 147 and 131).
 // CHIDG_STREAM_SHAPE="warps,stages,kbytes" overrides the sweeps' defaults
 // (comparison runs).
 namespace {
@@ -2206,20 +2214,24 @@ void init_shapes() {
     }
     for (int c = 0; c < kShapeClasses; ++c)
         for (int w = 0; w < 3; ++w) {
-            const StreamShape def{8, c == 0 ? 4 : 2, 26 * 1024};
-            g_shape[kShapeForward][c][w] = given ? sweep : StreamShape{8, def.nstage, 24 * 1024};
+            const StreamShape def{8, c == 0 ? 4 : 2, 26 * 1024, true};
+            g_shape[kShapeForward][c][w] = given ? sweep : StreamShape{8, def.nstage, 24 * 1024, true};
             g_shape[kShapeBackward][c][w] = given ? sweep : def;
             g_shape[kShapeBackwardMv][c][w] = def;
-            g_shape[kShapeMatvec][c][w] = StreamShape{8, 2, 24 * 1024};
+            g_shape[kShapeMatvec][c][w] = StreamShape{8, 2, 24 * 1024, true};
         }
     g_shape_init = true;
 }
 }  // namespace
 
-StreamShape chidg::stream_shape_for(int kind, int max_b, int esz) {
+StreamShape chidg::stream_shape_for(int kind, int max_b, int esz, bool diagonal) {
     std::lock_guard<std::mutex> lk(g_shape_mu);
     if (!g_shape_init) init_shapes();
-    return g_shape[kind][shape_class(max_b)][width_slot(esz)];
+    const int c = shape_class(max_b);
+    const StreamShape& sh = g_shape[kind][c][width_slot(esz)];
+    if (diagonal && sh.standard && kind == kShapeBackward) return StreamShape{8, 2, 24 * 1024, true};
+    if (diagonal && sh.standard && kind == kShapeBackwardMv && c == 0) return StreamShape{8, 2, 20 * 1024, true};
+    return sh;
 }
 void chidg::set_stream_shape(int kind, int max_b, int esz, const StreamShape& sh) {
     std::lock_guard<std::mutex> lk(g_shape_mu);
@@ -2311,7 +2323,7 @@ static int build_bwd_mv_tasks(chidg_gpu_precon* M, const chidg_gpu_matrix* A, in
         t.code = SW_MATVEC;
         t.b = P.prow_b[r];
         t.rbase = P.base_u[r];
-        t.nall = P.up[r].empty() ? 0 : P.whole_b[r] ? 1 : (int)P.up[r].size() * sweep_slices(t.b);
+        t.nall = P.up[r].empty() ? 0 : P.whole_b[r] ? 1 : (int)P.up[r].size() * P.slices(t.b);
         t.wait = -1;
         rows.push_back({4 * (last + 2 * lag) + 2, t});
     }
@@ -2371,7 +2383,7 @@ static int stream_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const T
     using ACC = typename AccOf<TV>::type;
     constexpr int esz = (int)sizeof(TL);
     const StreamShape sh = stream_shape_for(kShapeForward, P.max_b, esz);
-    const StreamShape shb = stream_shape_for(F ? kShapeBackwardMv : kShapeBackward, P.max_b, esz);
+    const StreamShape shb = stream_shape_for(F ? kShapeBackwardMv : kShapeBackward, P.max_b, esz, P.diagonal);
     Buffer& pb = (sizeof(ACC) == 8) ? M->part64 : M->part32;
     int st = ensure(ctx, pb, sizeof(ACC) * (size_t)P.part_s);
     if (st) return st;

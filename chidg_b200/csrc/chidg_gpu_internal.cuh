@@ -77,6 +77,8 @@ struct IluProgram {
     int64_t part_s = 0;
     int max_row_task_cols = 0;                 // widest segment a one-task row stages
     std::vector<uint8_t> whole_f, whole_b;     // rows that are one task
+    bool diagonal = false;                     // no couplings at all (Jacobi, precon_HB)
+    int slices(int b) const { return diagonal ? sweep_slices_diagonal(b) : sweep_slices(b); }
     bool no_lower = false;                     // no row has lower entries: the streamed forward sweep is left out
     std::vector<int64_t> base_f, base_u, base_d;
     Buffer d_sf_task, d_sb_task;
@@ -104,12 +106,13 @@ struct IluProgram {
 namespace chidg {
 // Launch shape of a streamed kernel: consumer warps, ring stages, bytes per
 // stage.  One shape per kernel kind, block-size class and value width: the
-// defaults below, or what the autotuner measured best (chidg_gpu_autotune).
-struct StreamShape { int cw = 8, nstage = 2, stage_bytes = 24 * 1024; };
+// defaults (other ones for programmes without couplings), or what the autotuner
+// measured best (chidg_gpu_autotune).
+struct StreamShape { int cw = 8, nstage = 2, stage_bytes = 24 * 1024; bool standard = false; };   // standard: a default
 enum { kShapeForward = 0, kShapeBackward = 1, kShapeBackwardMv = 2, kShapeMatvec = 3, kShapeKinds = 4 };
 constexpr int kShapeClasses = 4;                 // largest block: <= 64, <= 160, <= 384, <= 1024 rows
 inline int shape_class(int max_b) { return max_b <= 64 ? 0 : max_b <= 160 ? 1 : max_b <= 384 ? 2 : 3; }
-StreamShape stream_shape_for(int kind, int max_b, int esz);
+StreamShape stream_shape_for(int kind, int max_b, int esz, bool diagonal = false);
 void set_stream_shape(int kind, int max_b, int esz, const StreamShape& sh);
 // resident CTAs per SM of `func` (cached per function, block size and shared memory)
 int resident_ctas(const void* func, int threads, size_t smem);

@@ -40,8 +40,8 @@
 //   a task's indices come with its descriptor, not from dependent loads after
 //       the wait (an acquire leaves the SM's L1 without them).
 //
-// The cut depends on the row's own block size only, so a row sums in the same
-// order whatever matrix or batch it belongs to.
+// The cut depends on the row's own block size and on the kind of preconditioner
+// only, so a row sums in the same order whatever matrix or batch it belongs to.
 //
 // Bound by the copies at 24^3 elements of order 2 (5.8 and 15.8 GB: 1.14 ms
 // forward, 2.83 ms backward with matvec rows; with whole blocks as tasks 1.20 and
@@ -76,7 +76,19 @@ enum { SW_ENTRY = 0, SW_DIAG = 1, SW_ROW = 2, SW_MATVEC = 3 };   // slice of an 
 
 constexpr int SW_ROW_B = 64;      // rows of at most this size are one task (SW_ROW) ...
 constexpr int SW_ROW_COLS = 384;  // ... if their entries' columns fit the staged segment
-__host__ __device__ __forceinline__ int sweep_slices(int b) { return b <= SW_ROW_B ? 1 : b <= 160 ? 3 : 8; }
+inline int sweep_slices(int b) { return b <= SW_ROW_B ? 1 : b <= 160 ? 3 : 8; }
+// Programmes without couplings (Jacobi, precon_HB) have no chain, but the matvec
+// rows' wait.  Above 160 rows each of their slices is its own task however many
+// there are, which fills the last turn of the CTAs better than whole blocks (1 slice)
+// or grouped slices (8g); up to 256 rows eight are too many.  Apply, us, 1 / 3 / 8 /
+// 8g: 200 rows, 100 blocks 34 / 31 / 32 / 35, 720 73 / 70 / 85 / 82, 1500 106 / 107 /
+// 131 / 119; 320 rows, 100 blocks 55 / 44 / 42 / 43, 720 137 / 120 / 127 / 145, 1500
+// 218 / 211 / 222 / 231; 640 rows, 100 blocks 134 / 81 / 80 / 80, 990 559 / 490 / 509
+// / 586.  With the matvec rows eight are better than three above 256 rows (320 rows,
+// 60 blocks: 40 us a step).  At 135 rows ungrouped slices cost (1500 blocks 70 / 86;
+// grouped 75).
+inline int sweep_slices_diagonal(int b) { return b > 160 && b <= 256 ? 3 : sweep_slices(b); }
+inline bool sweep_groups_slices(int b, bool diagonal) { return !diagonal || b <= 160; }
 
 // A task.  A slice's (or several adjacent slices') staged segment is base[seg + c] -/+ the sum of npart
 // partial vectors part[pseg + k * pb + c] (pb: their row's size), c < cols:
@@ -92,7 +104,7 @@ struct alignas(16) StreamTask {
     int32_t par, wait;              // the wait: < 0 none, 0 flag of par, n its count reaching n
     int32_t npart, pb, src, nall;   // nall: tasks of the row (the last one completes it); SW_MATVEC, SW_ROW: U partial vectors of the row at rbase
     int32_t q0, q1;                 // the row's entries
-    int32_t nc, s0, nsl;            // slices s0 .. s0 + nsl - 1 of nc columns
+    int32_t nc, s0, nsl, ns;        // slices s0 .. s0 + nsl - 1 of the ns that nc columns are cut into
 };
 
 struct StreamMeta {
@@ -437,7 +449,7 @@ __global__ void __launch_bounds__(32 * CW + 32, CW == 16 ? 2 : CW == 8 ? 4 : 7) 
             } else {
                 const int esz = (FORWARD || d.code == SW_DIAG) ? (int)sizeof(TL) : (int)sizeof(TU);
                 // slices s0 .. s0 + nsl - 1 of the cut of nc columns, side by side
-                const int ns = sweep_slices(b);
+                const int ns = d.ns;
                 auto cut = [&](int s) { return d.nc * (d.s0 + s) / ns - d.nc * d.s0 / ns; };
                 for (int s = 0; s < d.nsl; ++s) nchunk += max(1, chunks(cut(s + 1) - cut(s), esz));
                 for (int s = 0; s < d.nsl; ++s) {

@@ -110,3 +110,27 @@ def test_inverses_of_many_large_blocks(sizes):
     with pytest.raises(_lib.ChidgGpuError) as ei:
         M.update(A)
     assert ei.value.code == _lib.ESINGULAR and ei.value.element == 77
+
+
+@pytest.mark.parametrize("count", [3, 310])
+@pytest.mark.parametrize("b", [64, 65, 160, 161, 256, 257, 385])
+def test_jacobi_apply_by_block_size(b, count):
+    """Slices of a programme without couplings: one task a row up to 64 rows,
+    three slices up to 160 (grouped from 296 blocks on) and up to 256 (never
+    grouped), eight above."""
+    rng = np.random.default_rng(66)
+    pat = mesh.box_pattern(count, 1, 1, 1, b)
+    voff, nval = pat.value_offsets()
+    diag = voff[np.asarray(pat.blk_face) == mesh.DIAG]
+    D = np.eye(b) + 0.5 / np.sqrt(b) * rng.uniform(-1.0, 1.0, (count, b, b))
+    vals = np.zeros(nval)
+    for o, d in zip(diag, D):
+        vals[o:o + b * b] = d.ravel(order="F")
+    v = rng.uniform(-1.0, 1.0, (count, b))
+    A = api.ChidgMatrix(pat)
+    A.upload(vals)
+    M = api.create_preconditioner("jacobi")
+    M.update(A)
+    z = M.apply(A, api.ChidgVector(A, v.ravel())).download().reshape(count, b)
+    tol = 64 * b * np.finfo(float).eps * max(np.linalg.cond(d) for d in D)
+    assert _relerr(z, np.linalg.solve(D, v[:, :, None])[:, :, 0]) < tol
