@@ -1306,6 +1306,14 @@ static void stream_layout(IluProgram& P) {
         }
         P.part_s = std::max(P.part_s, size);
     }
+    // the task-split schedule leaves one vector an entry in the same scratch:
+    // sized for both, so that a change of the schedule never moves it (captured
+    // sequences hold its address)
+    for (int fwd = 1; fwd >= 0; --fwd) {
+        int64_t size = 0;
+        for (int pr = 0; pr < np; ++pr) size += (int64_t)P.prow_b[pr] * (int64_t)(fwd ? P.lo : P.up)[pr].size();
+        P.part_s = std::max(P.part_s, size);
+    }
 }
 
 // Tasks in key order (those of one key as added): added once to count them and
@@ -2153,7 +2161,7 @@ static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV*
         M->tk_grid[variant] = std::max(1, per_sm * ctx->nsm);
     }
     Buffer& pb = (sizeof(ACC) == 8) ? M->part64 : M->part32;
-    int st = ensure(ctx, pb, sizeof(ACC) * (size_t)std::max<int64_t>(1, std::max(P.part_f, P.part_b)));
+    int st = ensure(ctx, pb, sizeof(ACC) * (size_t)P.part_s);
     if (st) return st;
     unsigned* sync = (unsigned*)M->sync.ptr;
     unsigned* flags = sync + 2;

@@ -253,3 +253,27 @@ print(json.dumps({"x": x.download().tolist(), "niter": [r["niter"] for r in res]
     assert s["hist"] == a["hist"]
     assert s["res"] == a["res"]
     assert np.array_equal(np.array(s["x"]), np.array(a["x"]))
+
+
+def test_replayed_steps_survive_a_change_of_schedule():
+    """Replayed Arnoldi steps hold the addresses of the sweeps' scratch: an
+    application with the task-split schedule in between must not move it."""
+    pats = [mesh.box_pattern(*s, 5, mesh.nterms_of_order(1)) for s in ((3, 3, 2), (4, 2, 2), (2, 3, 3))]
+    union, sys_elem = mesh.concat_patterns(pats)
+    A = api.ChidgMatrix(union)
+    A.upload(mesh.synth_values(union, seed=31))
+    b = api.ChidgVector(A, mesh.synth_vector(union.vector_size(), seed=32))
+    x = api.ChidgVector(A)
+    M = api.create_preconditioner("ilu0")
+    solver = api.create_linear_solver("fgmres", tol=0.0, rtol=1e-8, nkrylov=10, inner_fgmres=0, nmax=300)
+    for _ in range(4):
+        solver.solve_batched(A, x, b, M, sys_elem)
+    want = x.download()
+    z = M.apply(A, b).download()
+    M.set_schedule("tasks")
+    assert relerr(M.apply(A, b).download(), z) < 1e-12
+    others = [api.ChidgVector(A, np.full(union.vector_size(), np.nan)) for _ in range(8)]
+    M.set_schedule("stream")
+    solver.solve_batched(A, x, b, M, sys_elem)
+    assert np.array_equal(x.download(), want)
+    assert all(np.isnan(o.download()).all() for o in others)
