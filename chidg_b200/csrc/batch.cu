@@ -725,7 +725,7 @@ extern "C" int chidg_gpu_fgmres_solve_batched(chidg_gpu_matrix* A, chidg_gpu_pre
     // only the streamed sweeps clear their flags inside a captured sequence
     const bool sweeps_ok = M->kind == CHIDG_PRECON_IDENTITY ||
                            (M->schedule == CHIDG_SCHED_STREAM && M->P.max_b <= SS_MAX_B);
-    std::vector<int64_t> key = {A->uid, (int64_t)(intptr_t)M, (int64_t)M->kind, (int64_t)M->schedule, nsys, prec,
+    std::vector<int64_t> key = {A->uid, M->uid, (int64_t)M->kind, (int64_t)M->schedule, nsys, prec,
                                 (int64_t)(intptr_t)BB.cstart.ptr, (int64_t)M->P.nprow, M->P.ntask_bmv};
     key.insert(key.end(), sys_elem, sys_elem + nsys + 1);
 

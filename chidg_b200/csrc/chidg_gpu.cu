@@ -1739,6 +1739,8 @@ extern "C" int chidg_gpu_precon_create(chidg_gpu_matrix* A, int32_t kind, chidg_
     cudaSetDevice(ctx->device);
     if (kind < CHIDG_PRECON_IDENTITY || kind > CHIDG_PRECON_HB) return fail(ctx, CHIDG_GPU_EINVAL, "precon_create: unknown kind");
     auto* M = new chidg_gpu_precon();
+    static std::atomic<int64_t> next_uid{1};
+    M->uid = next_uid++;
     M->ctx = ctx;
     M->A = A;
     M->kind = kind;

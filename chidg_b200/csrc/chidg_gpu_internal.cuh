@@ -212,6 +212,7 @@ struct chidg_gpu_vector {
 };
 
 struct chidg_gpu_precon {
+    int64_t uid = 0;                       // unique over the process (captured sequences are kept by it, not by the address)
     chidg_gpu_ctx* ctx = nullptr;
     chidg_gpu_matrix* A = nullptr;
     int kind = 0;

@@ -277,3 +277,22 @@ def test_replayed_steps_survive_a_change_of_schedule():
     solver.solve_batched(A, x, b, M, sys_elem)
     assert np.array_equal(x.download(), want)
     assert all(np.isnan(o.download()).all() for o in others)
+
+
+def test_replayed_steps_are_not_those_of_an_earlier_preconditioner():
+    """A new preconditioner may get the address of one that was torn down."""
+    pats = [mesh.box_pattern(*s, 5, mesh.nterms_of_order(1), ntime=3) for s in ((2, 2, 2), (3, 2, 1))]
+    union, sys_elem = mesh.concat_patterns(pats)
+    A = api.ChidgMatrix(union)
+    A.upload(mesh.synth_values(union, seed=33))
+    b = api.ChidgVector(A, mesh.synth_vector(union.vector_size(), seed=34))
+    x = api.ChidgVector(A)
+    solver = api.create_linear_solver("fgmres", tol=0.0, rtol=1e-8, nkrylov=10, inner_fgmres=0, nmax=300)
+    want = None
+    for _ in range(3):
+        M = api.create_preconditioner("hb")
+        for _ in range(3):
+            solver.solve_batched(A, x, b, M, sys_elem)
+            want = x.download() if want is None else want
+            assert np.array_equal(x.download(), want)
+        M.tear_down()
