@@ -2803,6 +2803,7 @@ extern "C" int chidg_gpu_autotune(chidg_gpu_precon* M, chidg_gpu_matrix* A, int3
         const int max_b = kind == kShapeMatvec ? Aop->max_b : M->P.max_b;
         const int esz = kind == kShapeMatvec ? esz_matvec : esz_blocks;
         if (kind == kShapeMatvec && (Aop->max_b > SS_MAX_B || !Aop->rows_contiguous)) continue;
+        if (kind == kShapeForward && M->P.no_lower) continue;     // nothing runs: the class keeps its shape
         const StreamShape keep = stream_shape_for(kind, max_b, esz);
         StreamShape best = keep;
         float best_ms = 1e30f;

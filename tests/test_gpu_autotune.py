@@ -69,3 +69,16 @@ def test_shape_set_refuses_bad_shapes():
     assert L.chidg_gpu_stream_shape_set(0, 135, 8, 8, 1, 24576) == _lib.EINVAL      # stages
     assert L.chidg_gpu_stream_shape_set(0, 135, 3, 8, 2, 24576) == _lib.EINVAL      # value width
     assert L.chidg_gpu_stream_shape_set(9, 135, 8, 8, 2, 24576) == _lib.EINVAL      # kind
+
+
+def test_autotune_with_jacobi_leaves_the_forward_shape():
+    """Jacobi launches no forward sweep: there is nothing to measure, and the
+    shape of the class stays (ILU0 uses it)."""
+    pat, vals, _ = _system()
+    A = api.ChidgMatrix(pat)
+    A.upload(vals)
+    M = api.create_preconditioner("jacobi")
+    M.update(A)
+    before = tuning.get_shape(0, 135, 8)
+    assert tuning.autotune(A, M, "fp64", reps=1)["forward/b<=160/8B"] == before
+    assert tuning.get_shape(0, 135, 8) == before
