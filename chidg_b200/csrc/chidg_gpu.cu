@@ -17,6 +17,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <unordered_map>
 
@@ -301,13 +302,17 @@ extern "C" int chidg_gpu_host_free(void* p) {
 // chidg_matrix_t
 // ---------------------------------------------------------------------------
 template <typename T>
-static int upload_array(chidg_gpu_ctx* ctx, Buffer& buf, const std::vector<T>& v) {
-    int st = ensure(ctx, buf, std::max<size_t>(sizeof(T) * v.size(), sizeof(T)));
+static int upload_items(chidg_gpu_ctx* ctx, Buffer& buf, const T* v, size_t n) {
+    int st = ensure(ctx, buf, std::max<size_t>(sizeof(T) * n, sizeof(T)));
     if (st) return st;
-    if (v.empty()) return CHIDG_GPU_OK;
+    if (n == 0) return CHIDG_GPU_OK;
     // from pageable memory: staged before the call returns, so v may go
-    const cudaError_t e = cudaMemcpyAsync(buf.ptr, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, ctx->stream);
+    const cudaError_t e = cudaMemcpyAsync(buf.ptr, v, sizeof(T) * n, cudaMemcpyHostToDevice, ctx->stream);
     return e == cudaSuccess ? CHIDG_GPU_OK : cuda_fail(ctx, e, "pattern upload");
+}
+template <typename T>
+static int upload_array(chidg_gpu_ctx* ctx, Buffer& buf, const std::vector<T>& v) {
+    return upload_items(ctx, buf, v.data(), v.size());
 }
 
 // Triangular sweeps: one row per CTA and a dependency chain through the
@@ -1316,33 +1321,28 @@ static void stream_layout(IluProgram& P) {
     }
 }
 
-// Tasks in key order (those of one key as added): added once to count them and
-// once more, after place(), to be stored.
+// Tasks in key order (those of one key as added): their numbers first, then, after
+// place(), the tasks themselves, each written where it stays.
 struct KeyedTasks {
     int first;                        // the smallest key
     std::vector<int64_t> at;          // tasks of a key; then where its next one goes
-    std::vector<StreamTask> task;
-    bool placing = false;
+    std::unique_ptr<StreamTask[]> task;
+    int64_t n = 0;
     explicit KeyedTasks(int smallest) : first(smallest) {}
-    void add(int key, const StreamTask& t) {
+    void count(int key, int64_t tasks) {
         const size_t k = (size_t)(key - first);
-        if (placing) {
-            task[(size_t)at[k]++] = t;
-            return;
-        }
         if (at.size() <= k) at.resize(k + 1, 0);
-        ++at[k];
+        at[k] += tasks;
     }
     void place() {
-        int64_t n = 0;
         for (int64_t& a : at) {
             const int64_t here = a;
             a = n;
             n += here;
         }
-        task.resize((size_t)n);
-        placing = true;
+        task.reset(new StreamTask[(size_t)n]);    // (not zeroed: every one is written)
     }
+    StreamTask& next(int key) { return task[(size_t)at[(size_t)(key - first)]++]; }
 };
 
 // The tasks of a streamed sweep with their keys: a slice of an entry follows
@@ -1355,7 +1355,9 @@ struct KeyedTasks {
 // two an SM (24^3 of order 2, forward and backward sweep with matvec rows: 1139
 // and 2830 us; with four 1140 and 2938, with one 1164 and 2811, never 1430 and
 // 3145; 12^3: 260 and 491, 250 and 495, 296 and 523, 250 and 495).
-static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& lev, int scale, int many, KeyedTasks& keyed) {
+// With mv_key the matvec rows' tasks are among them, at these keys.
+static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& lev, int scale, int many, KeyedTasks& keyed,
+                         const std::vector<int>* mv_key = nullptr) {
     // blocks per level: inv(D) by the row's, entries by the parent's
     std::vector<int> dlev, elev;
     for (int pr = 0; pr < (int)P.prow_b.size(); ++pr) {
@@ -1370,6 +1372,22 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
     const std::vector<uint8_t>& whole = fwd ? P.whole_f : P.whole_b;
     std::vector<int> first(np + 1, 0);
     for (int pr = 0; pr < np; ++pr) first[pr + 1] = first[pr] + (int)(fwd ? P.lo : P.up)[pr].size();
+    // slices of a block that a task takes, by the blocks of its level
+    auto diag_step = [&](int pr, int b, int ns) { return dlev[lev[pr]] >= many && sweep_groups_slices(b, P.diagonal) ? ns : 1; };
+    auto entry_step = [&](int parent, int ns) { return elev[lev[parent]] >= many ? ns : 1; };
+    for (int pr = 0; pr < np; ++pr) {
+        const auto& ents = (fwd ? P.lo : P.up)[pr];
+        const int b = P.prow_b[pr], ns = P.slices(b);
+        if (mv_key) keyed.count((*mv_key)[pr], 1);
+        if (whole[pr]) {
+            keyed.count(scale * (2 * lev[pr] - 1), 1);
+            continue;
+        }
+        if (!fwd) keyed.count(scale * (2 * lev[pr] - 1), ns / diag_step(pr, b, ns));
+        for (const auto& en : ents) keyed.count(scale * (2 * lev[en.parent]), ns / entry_step(en.parent, ns));
+        if (fwd && ents.empty()) keyed.count(-scale, 1);
+    }
+    keyed.place();
     for (int32_t pr : fwd ? P.fwd_rows : P.bwd_rows) {
         const auto& ents = (fwd ? P.lo : P.up)[pr];
         const int b = P.prow_b[pr], ns = P.slices(b), ne = (int)ents.size();
@@ -1391,13 +1409,14 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
             t.out = t.rbase = fwd ? 0 : P.base_u[pr];
             t.nall = ne ? 1 : 0;
             t.src = !fwd && P.lo[pr].empty();
-            keyed.add(scale * (2 * lev[pr] - 1), t);
+            keyed.next(scale * (2 * lev[pr] - 1)) = t;
             continue;
         }
-        const int dstep = dlev[lev[pr]] >= many && sweep_groups_slices(b, P.diagonal) ? ns : 1;
+        const int dstep = diag_step(pr, b, ns);
         if (!fwd)
             for (int s = 0; s < ns; s += dstep) {
-                StreamTask u = t;
+                StreamTask& u = keyed.next(scale * (2 * lev[pr] - 1));
+                u = t;
                 u.nc = b;
                 u.s0 = s;
                 u.nsl = dstep;
@@ -1414,12 +1433,12 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
                 u.src = P.lo[pr].empty();
                 u.seg = (u.src ? t.vrow : t.zrow) + c0;
                 u.pseg = P.base_u[pr] + c0;
-                keyed.add(scale * (2 * lev[pr] - 1), u);
             }
         for (int e = 0; e < ne; ++e) {
-            const int step = elev[lev[ents[e].parent]] >= many ? ns : 1;
+            const int step = entry_step(ents[e].parent, ns);
             for (int s = 0; s < ns; s += step) {
-                StreamTask u = t;
+                StreamTask& u = keyed.next(scale * (2 * lev[ents[e].parent]));
+                u = t;
                 u.nc = ents[e].nc;
                 u.s0 = s;
                 u.nsl = step;
@@ -1449,19 +1468,29 @@ static void stream_tasks(const IluProgram& P, bool fwd, const std::vector<int>& 
                     u.src = 2;
                     u.pseg = P.base_d[q] + c0;
                 }
-                keyed.add(scale * (2 * lev[q]), u);
             }
         }
         if (fwd && ne == 0) {
             // z_r = v_r for whoever reads it (the backward sweep): a slice of no columns
-            StreamTask u = t;
+            StreamTask& u = keyed.next(-scale);
+            u = t;
             u.code = SW_ENTRY;
             u.rbase = u.out = P.base_f[pr];
             u.nall = 1;
             u.nsl = 1;
-            keyed.add(-scale, u);
         }
     }
+    if (mv_key)
+        for (int r = 0; r < np; ++r) {
+            StreamTask& t = keyed.next((*mv_key)[r]);
+            t = StreamTask{};
+            t.row = r;
+            t.code = SW_MATVEC;
+            t.b = P.prow_b[r];
+            t.rbase = P.base_u[r];
+            t.nall = P.up[r].empty() ? 0 : P.whole_b[r] ? 1 : (int)P.up[r].size() * P.slices(t.b);
+            t.wait = -1;
+        }
 }
 
 // Levels, LD slots, GEMM tasks, device upload.
@@ -1501,47 +1530,6 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
     bucket(lb, P.bwd_rows, P.bwd_ptr);
     P.lb = lb;
     P.bmv_uid = -1;
-    // task-split sweeps: one task per entry, combine-only tasks for rows
-    // without entries; hand-out order by the level of the parent row
-    {
-        auto build_tasks = [&](bool fwd, std::vector<int32_t>& trow, std::vector<int32_t>& tent,
-                               std::vector<int64_t>& poff, int64_t& psize) {
-            const std::vector<int32_t>& order = fwd ? P.fwd_rows : P.bwd_rows;
-            const std::vector<int>& lev = fwd ? lf : lb;
-            std::vector<std::pair<int, std::pair<int32_t, int32_t>>> keyed;
-            int base = 0;
-            std::vector<int> first(np, 0);
-            for (int pr = 0; pr < np; ++pr) { first[pr] = base; base += (int)(fwd ? P.lo[pr].size() : P.up[pr].size()); }
-            poff.assign(base, 0);
-            psize = 0;
-            for (int pr = 0; pr < np; ++pr) {
-                const auto& ents = fwd ? P.lo[pr] : P.up[pr];
-                for (size_t e = 0; e < ents.size(); ++e) { poff[first[pr] + e] = psize; psize += P.prow_b[pr]; }
-            }
-            for (int32_t pr : order) {
-                const auto& ents = fwd ? P.lo[pr] : P.up[pr];
-                if (ents.empty()) keyed.push_back({-1, {pr, -1}});
-                for (size_t e = 0; e < ents.size(); ++e) keyed.push_back({lev[ents[e].parent], {pr, first[pr] + (int32_t)e}});
-            }
-            std::stable_sort(keyed.begin(), keyed.end(), [](const auto& a, const auto& c) { return a.first < c.first; });
-            trow.clear();
-            tent.clear();
-            for (auto& k : keyed) { trow.push_back(k.second.first); tent.push_back(k.second.second); }
-        };
-        std::vector<int32_t> tr, te;
-        std::vector<int64_t> po;
-        int st0;
-        build_tasks(true, tr, te, po, P.part_f);
-        P.ntask_f = (int)tr.size();
-        if ((st0 = upload_array(ctx, P.d_tf_row, tr)) || (st0 = upload_array(ctx, P.d_tf_ent, te)) ||
-            (st0 = upload_array(ctx, P.d_poff_f, po)))
-            return st0;
-        build_tasks(false, tr, te, po, P.part_b);
-        P.ntask_b = (int)tr.size();
-        if ((st0 = upload_array(ctx, P.d_tb_row, tr)) || (st0 = upload_array(ctx, P.d_tb_ent, te)) ||
-            (st0 = upload_array(ctx, P.d_poff_b, po)))
-            return st0;
-    }
     // LD slots: per programme row [inv(D)][L_1][L_2]...
     P.dinv_off.assign(np, 0);
     int64_t ld = 0;
@@ -1556,13 +1544,10 @@ static int finalize_program(chidg_gpu_ctx* ctx, const chidg_gpu_matrix* A, IluPr
     stream_layout(P);
     for (int fwd = 1; fwd >= 0; --fwd) {
         KeyedTasks keyed(-1);
-        for (int pass = 0; pass < 2; ++pass) {
-            stream_tasks(P, fwd != 0, fwd ? lf : lb, 1, 2 * ctx->nsm, keyed);
-            if (pass == 0) keyed.place();
-        }
+        stream_tasks(P, fwd != 0, fwd ? lf : lb, 1, 2 * ctx->nsm, keyed);
         int st0;
-        if ((st0 = upload_array(ctx, fwd ? P.d_sf_task : P.d_sb_task, keyed.task))) return st0;
-        (fwd ? P.ntask_sf : P.ntask_sb) = (int)keyed.task.size();
+        if ((st0 = upload_items(ctx, fwd ? P.d_sf_task : P.d_sb_task, keyed.task.get(), (size_t)keyed.n))) return st0;
+        (fwd ? P.ntask_sf : P.ntask_sb) = (int)keyed.n;
     }
     // flatten entry lists
     std::vector<int32_t> lo_ptr(np + 1, 0), up_ptr(np + 1, 0), lo_par, up_par, lo_nc, up_nc;
@@ -2136,6 +2121,43 @@ static int dataflow_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const
     return CHIDG_GPU_OK;
 }
 
+// The task-split sweeps' lists, built when that schedule first runs: one task per
+// entry, combine-only tasks for rows without entries; hand-out order by the
+// level of the parent row.
+static int build_split_tasks(chidg_gpu_ctx* ctx, IluProgram& P) {
+    if (P.d_tf_row.ptr != nullptr) return CHIDG_GPU_OK;
+    const int np = P.nprow;
+    std::vector<int> lf(np, 0);
+    for (int l = 0; l + 1 < (int)P.fwd_ptr.size(); ++l)
+        for (int i = P.fwd_ptr[l]; i < P.fwd_ptr[l + 1]; ++i) lf[P.fwd_rows[i]] = l;
+    for (int fwd = 0; fwd < 2; ++fwd) {
+        const std::vector<int>& lev = fwd ? lf : P.lb;
+        std::vector<std::pair<int, std::pair<int32_t, int32_t>>> keyed;
+        std::vector<int> first(np + 1, 0);
+        for (int pr = 0; pr < np; ++pr) first[pr + 1] = first[pr] + (int)(fwd ? P.lo : P.up)[pr].size();
+        std::vector<int64_t> poff(first[np]);
+        int64_t psize = 0;
+        for (int pr = 0; pr < np; ++pr)
+            for (int e = first[pr]; e < first[pr + 1]; ++e) { poff[e] = psize; psize += P.prow_b[pr]; }
+        for (int32_t pr : fwd ? P.fwd_rows : P.bwd_rows) {
+            const auto& ents = (fwd ? P.lo : P.up)[pr];
+            if (ents.empty()) keyed.push_back({-1, {pr, -1}});
+            for (size_t e = 0; e < ents.size(); ++e) keyed.push_back({lev[ents[e].parent], {pr, first[pr] + (int32_t)e}});
+        }
+        std::stable_sort(keyed.begin(), keyed.end(), [](const auto& a, const auto& c) { return a.first < c.first; });
+        std::vector<int32_t> row, ent;
+        for (auto& k : keyed) { row.push_back(k.second.first); ent.push_back(k.second.second); }
+        (fwd ? P.ntask_f : P.ntask_b) = (int)row.size();
+        int st;
+        // (the forward rows last: they say that the lists are there)
+        if ((st = upload_array(ctx, fwd ? P.d_poff_f : P.d_poff_b, poff)) ||
+            (st = upload_array(ctx, fwd ? P.d_tf_ent : P.d_tb_ent, ent)) ||
+            (st = upload_array(ctx, fwd ? P.d_tf_row : P.d_tb_row, row)))
+            return st;
+    }
+    return CHIDG_GPU_OK;
+}
+
 // Both sweeps as two task-split launches (CHIDG_SCHED_TASKS).
 template <typename TL, typename TU, typename TV>
 static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV* v, TV* zx, int variant) {
@@ -2164,7 +2186,7 @@ static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV*
     }
     Buffer& pb = (sizeof(ACC) == 8) ? M->part64 : M->part32;
     int st = ensure(ctx, pb, sizeof(ACC) * (size_t)P.part_s);
-    if (st) return st;
+    if (st || (st = build_split_tasks(ctx, P))) return st;
     unsigned* sync = (unsigned*)M->sync.ptr;
     unsigned* flags = sync + 2;
     SweepSync S{sync, flags, 0u, (int*)(ctx->d_scal + kSlotStatus), kSpinLimit};
@@ -2303,8 +2325,8 @@ static int stream_launch(chidg_gpu_precon* M, const TL* LD, const TU* U, StreamT
 static int build_bwd_mv_tasks(chidg_gpu_precon* M, const chidg_gpu_matrix* A, int lag) {
     IluProgram& P = M->P;
     if (P.bmv_uid == A->uid && P.bmv_lag == lag) return CHIDG_GPU_OK;
-    std::vector<std::pair<int, StreamTask>> rows;
-    rows.reserve((size_t)A->nrow);
+    std::vector<int> mv_key;
+    mv_key.reserve((size_t)A->nrow);
     std::vector<int32_t> col_prow;
     col_prow.reserve(A->nblk);
     // the matrix blocks that are the sweep's U blocks (same values, same
@@ -2328,27 +2350,16 @@ static int build_bwd_mv_tasks(chidg_gpu_precon* M, const chidg_gpu_matrix* A, in
             skip.push_back(u);
         }
         if (matched != (int)P.up[r].size()) reuse = false;
-        StreamTask t{};
-        t.row = r;
-        t.code = SW_MATVEC;
-        t.b = P.prow_b[r];
-        t.rbase = P.base_u[r];
-        t.nall = P.up[r].empty() ? 0 : P.whole_b[r] ? 1 : (int)P.up[r].size() * P.slices(t.b);
-        t.wait = -1;
-        rows.push_back({4 * (last + 2 * lag) + 2, t});
+        mv_key.push_back(4 * (last + 2 * lag) + 2);
     }
     KeyedTasks keyed(-4);
-    for (int pass = 0; pass < 2; ++pass) {
-        stream_tasks(P, false, P.lb, 4, 2 * M->ctx->nsm, keyed);
-        for (const auto& r : rows) keyed.add(r.first, r.second);
-        if (pass == 0) keyed.place();
-    }
+    stream_tasks(P, false, P.lb, 4, 2 * M->ctx->nsm, keyed, &mv_key);
     int st;
-    if ((st = upload_array(M->ctx, P.d_bmv_task, keyed.task)) || (st = upload_array(M->ctx, P.d_col_prow, col_prow)) ||
+    if ((st = upload_items(M->ctx, P.d_bmv_task, keyed.task.get(), (size_t)keyed.n)) || (st = upload_array(M->ctx, P.d_col_prow, col_prow)) ||
         (st = upload_array(M->ctx, P.d_mv_skip, skip)))
         return st;
     P.bmv_reuse = reuse;
-    P.ntask_bmv = (int)keyed.task.size();
+    P.ntask_bmv = (int)keyed.n;
     P.bmv_uid = A->uid;
     P.bmv_lag = lag;
     return CHIDG_GPU_OK;

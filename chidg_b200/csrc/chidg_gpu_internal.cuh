@@ -67,9 +67,8 @@ struct IluProgram {
     std::vector<int> ltask_ptr, stask_ptr;      // factor products per level
     std::vector<int> ltask_small, stask_small;  // of them, those the FP32 kernels for small blocks take (first in the level)
     std::vector<std::array<int, 3>> inv_seg;   // per level: (row_begin, count, largest block)
-    // task-split sweeps: tasks in hand-out order, partial offsets per entry
+    // task-split sweeps (built at their first run): tasks in hand-out order, partial offsets per entry
     int ntask_f = 0, ntask_b = 0;
-    int64_t part_f = 0, part_b = 0;            // scratch sizes (values)
     Buffer d_tf_row, d_tf_ent, d_tb_row, d_tb_ent, d_poff_f, d_poff_b;
     // streamed sweeps: tasks (StreamTask), partial sums (the two sweeps use the
     // same scratch), the first partials of every row's entries and of inv(D)
