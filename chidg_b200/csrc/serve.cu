@@ -18,6 +18,7 @@
 #include "chidg_gpu_internal.cuh"
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -98,11 +99,12 @@ namespace {
 
 // Device bytes one request needs: its blocks (nval values), the ILU factors
 // (the values of its diagonal and lower blocks, nlow), their FP32 copies in a
-// mixed mode, the Krylov basis and a few vectors.  An estimate for admission:
-// a batch that does not fit after all is solved in halves.
-int64_t request_bytes(int64_t nval, int64_t nlow, int64_t n, int32_t nkrylov, int32_t precision) {
+// mixed mode, the sweeps' scratch and tasks (nsweep bytes), the Krylov basis and a
+// few vectors.  An estimate for admission: a batch that does not fit after all is
+// solved in halves.
+int64_t request_bytes(int64_t nval, int64_t nlow, int64_t nsweep, int64_t n, int32_t nkrylov, int32_t precision) {
     const int64_t blocks = 8 * (nval + nlow) + (precision != CHIDG_GPU_FP64 ? 4 * (nval + nlow) : 0);
-    return blocks + 8 * n * (2 * ((int64_t)nkrylov + 1) + 6);
+    return blocks + nsweep + 8 * n * (2 * ((int64_t)nkrylov + 1) + 6);
 }
 
 // Solve requests [first, last) of a batch as one packed system on ctx; on
@@ -377,16 +379,24 @@ std::shared_ptr<Request> new_request(const chidg_gpu_server* S, const chidg_gpu_
         q->n += (int64_t)pat->ntime * q->nvars[e] * q->nterms[e];
     }
     int64_t nlow = 0;                        // values of the diagonal and lower blocks (natural order)
+    std::vector<std::array<int, 2>> rows((size_t)ne * pat->ntime, {0, 0});   // lower and upper entries of every row
     for (int64_t k = 0; k < nb; ++k) {
         if (q->re[k] < 0 || q->re[k] >= ne || q->ce[k] < 0 || q->ce[k] >= ne) return nullptr;
         const int64_t v = (int64_t)q->nvars[q->re[k]] * q->nterms[q->re[k]] * q->nvars[q->ce[k]] * q->nterms[q->ce[k]];
         q->nval += v;
         if (q->ce[k] < q->re[k] || (q->ce[k] == q->re[k] && q->ct[k] <= q->rt[k])) nlow += v;
+        if (q->ce[k] != q->re[k] && q->rt[k] >= 0 && q->rt[k] < pat->ntime)
+            ++rows[(size_t)q->re[k] * pat->ntime + q->rt[k]][q->ce[k] > q->re[k]];
+    }
+    int64_t nsweep = 0;
+    for (size_t r = 0; r < rows.size(); ++r) {
+        const size_t e = r / pat->ntime;
+        nsweep += chidg::sweep_row_bytes(q->nvars[e] * q->nterms[e], rows[r][0], rows[r][1]);
     }
     q->pat.nelem = pat->nelem;               // the arrays are copied above; keep only the sizes
     q->pat.ntime = pat->ntime;
     q->pat.nblocks = pat->nblocks;
-    q->bytes = request_bytes(q->nval, nlow, q->n, S->opts.nkrylov, S->opts.precision);
+    q->bytes = request_bytes(q->nval, nlow, nsweep, q->n, S->opts.nkrylov, S->opts.precision);
     return q;
 }
 

@@ -62,6 +62,8 @@
 // bytes of slack past their end, so the rounded copies stay inside them.
 #pragma once
 
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace chidg {
@@ -106,6 +108,15 @@ struct alignas(16) StreamTask {
     int32_t q0, q1;                 // the row's entries
     int32_t nc, s0, nsl, ns;        // slices s0 .. s0 + nsl - 1 of the ns that nc columns are cut into
 };
+
+// Device bytes that a row of nlo lower and nup upper entries adds to the sweeps'
+// scratch and task lists, at most (the forward, the backward and the list with the
+// matvec row)
+inline int64_t sweep_row_bytes(int b, int nlo, int nup) {
+    const int64_t ns = sweep_slices(b), task = sizeof(StreamTask);
+    if (b <= SW_ROW_B) return 8 * (int64_t)b * std::max(nlo, nup) + 4 * task;
+    return 8 * b * ns * std::max(nlo, nup + 1) + task * (ns * (nlo + 2 * (nup + 1)) + 2);
+}
 
 struct StreamMeta {
     int task;      // descriptor slot, -1 = end of the sweep for this CTA

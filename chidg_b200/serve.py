@@ -67,7 +67,7 @@ def request_bytes(pat: mesh.BlockPattern, nkrylov: int, precision: str = "fp64")
     """Device bytes one request needs (an estimate for admission, as the
     native server makes it): its blocks, the ILU factors (the values of the
     diagonal and lower blocks in natural order), their FP32 copies in a mixed
-    mode, the Krylov basis and a few vectors."""
+    mode, the sweeps' scratch and tasks, the Krylov basis and a few vectors."""
     _, nval = pat.value_offsets()
     nr, nc = pat.block_dims()
     re, ce = np.asarray(pat.blk_row_elem), np.asarray(pat.blk_col_elem)
@@ -76,7 +76,15 @@ def request_bytes(pat: mesh.BlockPattern, nkrylov: int, precision: str = "fp64")
     nlow = int((np.asarray(nr, dtype=np.int64) * np.asarray(nc, dtype=np.int64))[low].sum())
     n = pat.vector_size()
     blocks = 8 * (nval + nlow) + (4 * (nval + nlow) if precision != "fp64" else 0)
-    return int(blocks + 8 * n * (2 * (nkrylov + 1) + 6))
+    # sweep_row_bytes of csrc/stream_sweep.cuh, row by row
+    row = re * pat.ntime + rt
+    nlo = np.bincount(row[ce < re], minlength=pat.nelem * pat.ntime)
+    nup = np.bincount(row[ce > re], minlength=pat.nelem * pat.ntime)
+    b = np.repeat(pat.bsize(), pat.ntime)
+    ns = np.where(b <= 160, 3, 8)
+    sweeps = np.where(b <= 64, 8 * b * np.maximum(nlo, nup) + 4 * 128,
+                      8 * b * ns * np.maximum(nlo, nup + 1) + 128 * (ns * (nlo + 2 * (nup + 1)) + 2))
+    return int(blocks + sweeps.sum() + 8 * n * (2 * (nkrylov + 1) + 6))
 
 
 class Server:
