@@ -488,7 +488,6 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
     double* sFs = sFI + (size_t)6 * qf * 5;     // [6][qf][5][5]  d integrand / d own state
     double* sFn = sFs + (size_t)6 * qf * 25;    // [6][qf][5][5]  d integrand / d neighbour state
     constexpr int RT = row_tiles(NT), CT = col_tiles(NT), ITEMS = row_items(NT);
-    const int warp = threadIdx.x >> 5;
     __shared__ int sFaces[6], sNext;            // faces with a neighbour; next item of the blocks
     int nbr[6], nface = 0;
 #pragma unroll
@@ -500,13 +499,6 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
         }
     }
     if (threadIdx.x == 0) sNext = 0;
-    auto next_item = [&]() {
-        int it = 0;
-        if ((threadIdx.x & 31) == 0) it = atomicAdd(&sNext, 1);
-        return __shfl_sync(0xffffffffu, it, 0);
-    };
-    (void)warp;
-    (void)next_item;
 
     // 1. modes of the element and its neighbours
     for (int t = threadIdx.x; t < 7 * b; t += blockDim.x) {
@@ -545,11 +537,12 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
         // warps take items (a block, RT row tiles of it) as they come free,
         // the DIAG block's, which are the long ones, first
         if (val == nullptr) return;
-        const int* face_of = sFaces;
         for (;;) {
-            const int it = next_item();
+            int it = 0;
+            if ((threadIdx.x & 31) == 0) it = atomicAdd(&sNext, 1);
+            it = __shfl_sync(0xffffffffu, it, 0);
             if (it >= (1 + nface) * ITEMS) break;
-            const int blk = it < ITEMS ? 6 : face_of[it / ITEMS - 1], rt0 = (it % ITEMS) * RT;
+            const int blk = it < ITEMS ? 6 : sFaces[it / ITEMS - 1], rt0 = (it % ITEMS) * RT;
             double acc[RT][5][CT][2];
             clear_tiles<NT, RT>(acc);
             if (blk == 6) {
@@ -571,6 +564,7 @@ __global__ void __launch_bounds__(kThreads) k_euler_assemble(BoxGeom g, Tables t
         // continues them (each output value is read back by the thread that
         // wrote it).
         const int64_t* bo = blk_off + (int64_t)e * 7;
+        const int warp = threadIdx.x >> 5;
         // ---- volume pass
         for (int t = threadIdx.x; t < qv; t += blockDim.x) volume_node<NT>(tb, sU, t, nt, sWF, sWdF);
         __syncthreads();
