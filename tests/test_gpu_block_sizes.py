@@ -1,8 +1,11 @@
 """Factorisation and sweeps at the block sizes where their kernels change
 shape: the factor products' tiles (8 x 8 accumulators, CTA tiles of at most 80
-x 80), the inverses' panels of eight, row pairs of sixteen and cluster sizes
-(one CTA up to 136 rows, more above, another kernel above 384), the sweeps'
-one-task rows (up to 64) and column slices (three up to 160, eight above)."""
+x 80), the inverses' panels of eight, row pairs of sixteen and cluster sizes (one
+CTA up to 152 rows, two up to 208, three up to 256, four up to 288, five up to
+320, six up to 352, seven up to 384, another kernel above), the sweeps' one-task
+rows (up to 64) and column slices (three up to 160, eight above); matrices that
+mix those sizes; and the sweeps' tasks where a level has blocks enough for a task
+to take all slices of one."""
 import numpy as np
 import pytest
 
@@ -12,8 +15,9 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 # (fields, modes): block size is their product
-SIZES = [(1, 1), (7, 1), (1, 8), (3, 3), (5, 8), (13, 5), (8, 10), (27, 3), (1, 127), (17, 8), (1, 137), (32, 5), (7, 23),
-         (13, 16), (11, 19), (7, 40), (64, 5), (3, 107), (128, 3), (5, 77)]
+SIZES = [(1, 1), (7, 1), (1, 8), (3, 3), (5, 8), (13, 5), (8, 10), (27, 3), (1, 127), (17, 8), (1, 137), (8, 19), (9, 17),
+         (32, 5), (7, 23), (13, 16), (11, 19), (4, 64), (1, 257), (7, 40), (36, 8), (17, 17), (64, 5), (3, 107), (44, 8),
+         (1, 353), (128, 3), (5, 77)]
 
 
 def _relerr(a, b):
@@ -134,3 +138,83 @@ def test_jacobi_apply_by_block_size(b, count):
     z = M.apply(A, api.ChidgVector(A, v.ravel())).download().reshape(count, b)
     tol = 64 * b * np.finfo(float).eps * max(np.linalg.cond(d) for d in D)
     assert _relerr(z, np.linalg.solve(D, v[:, :, None])[:, :, 0]) < tol
+
+
+def _mixed(pat, sizes, seed):
+    """The pattern with one field and a block size from `sizes` per element, its
+    values, and the oracle's and the library's matrices."""
+    pat.elem_nterms[:] = np.random.default_rng(seed).choice(sizes, pat.nelem)
+    vals = mesh.synth_values(pat, seed=seed)
+    Ao, Ag = O.OracleMatrix(pat), api.ChidgMatrix(pat)
+    Ao.set_values(vals)
+    Ag.upload(vals)
+    return vals, Ao, Ag
+
+
+@pytest.mark.parametrize("sizes", [(40, 135, 320), (64, 65, 160, 161), (135, 320), (209, 243, 320), (321, 350, 384)],
+                         ids=lambda s: "-".join(map(str, s)))
+def test_mixed_block_sizes(sizes):
+    """Rows of one, three and eight slices next to one another, and inverses of
+    different sizes in one launch: factors, an application and a solve with the
+    matvec rows in the backward sweep, against the oracle.  Tolerances as in
+    test_gpu_edge.py."""
+    pat = mesh.box_pattern(3, 3, 2, 1, sizes[0])
+    vals, Ao, Ag = _mixed(pat, sizes, 71)
+    Mo, Mg = O.OraclePrecon(Ao, "ilu0"), api.create_preconditioner("ilu0")
+    Mo.update()
+    Mg.update(Ag)
+    voff, _ = pat.value_offsets()
+    nr, nc = pat.block_dims()
+    LDo, LDg = Mo.LD(), Mg.LD()
+    for k in range(pat.nblocks):
+        o = LDo[voff[k]:voff[k] + nr[k] * nc[k]]
+        if np.any(o):
+            assert _relerr(LDg[voff[k]:voff[k] + nr[k] * nc[k]], o) < 1e-10
+    v = mesh.synth_vector(pat.vector_size(), seed=72)
+    assert _relerr(Mg.apply(Ag, api.ChidgVector(Ag, v)).download(), Mo.apply(v)) < 1e-11
+    opts = dict(tol=0.0, rtol=1e-8, nkrylov=20, inner_fgmres=0, nmax=400)
+    xo, ro = O.fgmres(Ao, O.OraclePrecon(Ao, "ilu0"), v, O.default_opts(**opts))
+    x, solver = api.ChidgVector(Ag), api.create_linear_solver("fgmres", **opts)
+    solver.solve(Ag, x, api.ChidgVector(Ag, v), Mg)
+    assert solver.niter == ro["niter"]
+    assert _relerr(x.download(), xo) < 1e-10
+
+
+def test_product_of_mixed_sizes_with_more_rows_than_ctas():
+    """1716 rows of 5 and 40 equations: the rows by falling size, several turns of
+    the CTAs."""
+    pat = mesh.with_element_orders(mesh.box_pattern(11, 13, 12, 5, 8), np.random.default_rng(73).integers(0, 2, 1716))
+    vals = mesh.synth_values(pat, seed=74)
+    Ao, Ag = O.OracleMatrix(pat), api.ChidgMatrix(pat)
+    Ao.set_values(vals)
+    Ag.upload(vals)
+    x = mesh.synth_vector(pat.vector_size(), seed=75)
+    assert _relerr(api.chidg_mv(Ag, api.ChidgVector(Ag, x)).download(), Ao.mv(x)) < 1e-13
+
+
+@pytest.mark.parametrize("b", [65, 161])
+def test_grouped_slices_give_the_sums_of_single_ones(b):
+    """300 systems side by side: levels of 300 blocks, whose tasks take all three
+    (65 rows) or eight (161) slices of a block.  Bitwise the application of a
+    system alone, whose tasks take a slice each; one of them against the oracle."""
+    one = mesh.box_pattern(2, 1, 1, 1, b)
+    union, sys_elem = mesh.concat_patterns([one] * 300)
+    vals = np.concatenate([mesh.synth_values(one, seed=80 + s % 7) for s in range(300)])
+    v = mesh.synth_vector(union.vector_size(), seed=81)
+    A = api.ChidgMatrix(union)
+    A.upload(vals)
+    M = api.create_preconditioner("ilu0")
+    M.update(A)
+    z = M.apply(A, api.ChidgVector(A, v)).download().reshape(300, -1)
+    v = v.reshape(300, -1)
+    for s in (0, 1, 150, 299):
+        A1 = api.ChidgMatrix(one)
+        A1.upload(mesh.synth_values(one, seed=80 + s % 7))
+        M1 = api.create_preconditioner("ilu0")
+        M1.update(A1)
+        assert np.array_equal(z[s], M1.apply(A1, api.ChidgVector(A1, v[s])).download())
+    Ao = O.OracleMatrix(one)
+    Ao.set_values(mesh.synth_values(one, seed=80))
+    Mo = O.OraclePrecon(Ao, "ilu0")
+    Mo.update()
+    assert _relerr(z[0], Mo.apply(v[0])) < 1e-11
