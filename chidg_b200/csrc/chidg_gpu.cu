@@ -2299,7 +2299,13 @@ static int stream_launch(chidg_gpu_precon* M, const TL* LD, const TU* U, StreamT
     if ((size_t)sh.stage_bytes < (size_t)M->P.max_b * std::max(sizeof(TL), sizeof(TU)) + 16 ||
         (MV && (size_t)sh.stage_bytes < (size_t)M->P.max_b * sizeof(TA) + 16))
         return fail(ctx, CHIDG_GPU_EINVAL, "streamed sweep: stage smaller than one block column");
-    const size_t smem = stream_smem_bytes(sizeof(ACC), sh.nstage, sh.stage_bytes, xcols, 32 * CW);
+    // a default ring gives way to a very wide staged segment (a row of some 200 blocks)
+    constexpr size_t kMostSmem = 226 * 1024;         // beside the kernel's own few hundred bytes
+    StreamShape ring = sh;
+    auto bytes = [&]() { return stream_smem_bytes(sizeof(ACC), ring.nstage, ring.stage_bytes, xcols, 32 * CW); };
+    while (ring.standard && bytes() > kMostSmem && ring.nstage > 2) --ring.nstage;
+    if (ring.standard && bytes() > kMostSmem) ring.stage_bytes = std::min(ring.stage_bytes, 20 * 1024);
+    const size_t smem = bytes();
     auto k = k_ilu_stream<TL, TU, TV, ACC, FWD, CW, TA, MV>;
     int st;
     if ((st = raise_smem_limit((const void*)k, smem))) return fail(ctx, st, "streamed sweep shared memory");
@@ -2311,7 +2317,7 @@ static int stream_launch(chidg_gpu_precon* M, const TL* LD, const TU* U, StreamT
     const bool rows_match = (M->kind == CHIDG_PRECON_ILU0 || M->kind == CHIDG_PRECON_JACOBI) && M->P.nprow == ctx->row_mask.nrow;
     const RowMask mk = rows_match ? ctx->row_mask : RowMask{};
     k<<<std::max(1, std::min(grid, ntask)), 32 * CW + 32, smem, ctx->stream>>>(M->P.rows, LD, U, Tk, ntask, v, zx, (ACC*)part,
-                                                                              S, sh.nstage, sh.stage_bytes, xcols, F, mk);
+                                                                              S, ring.nstage, ring.stage_bytes, xcols, F, mk);
     return check_launch(ctx, MV ? "k_ilu_stream backward + matvec" : FWD ? "k_ilu_stream forward" : "k_ilu_stream backward");
 }
 

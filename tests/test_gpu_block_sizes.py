@@ -218,3 +218,20 @@ def test_grouped_slices_give_the_sums_of_single_ones(b):
     Mo = O.OraclePrecon(Ao, "ilu0")
     Mo.update()
     assert _relerr(z[0], Mo.apply(v[0])) < 1e-11
+
+
+def test_rows_of_very_many_blocks():
+    """One element with 240 time levels of 64 equations: the matvec rows of the
+    backward sweep stage 15 360 columns, beside which four stages of the default
+    ring do not fit.  Against the sweeps without matvec rows."""
+    pat = mesh.box_pattern(1, 1, 1, 8, 8, ntime=240)
+    A = api.ChidgMatrix(pat)
+    A.upload(mesh.synth_values(pat, seed=91))
+    b = api.ChidgVector(A, mesh.synth_vector(pat.vector_size(), seed=92))
+    xs = []
+    for schedule in ("stream", "levels"):
+        x = api.ChidgVector(A)
+        solver = api.create_linear_solver("fgmres", tol=0.0, rtol=1e-30, nkrylov=4, nmax=4, inner_fgmres=0)
+        solver.solve(A, x, b, api.create_preconditioner("ilu0", schedule=schedule))
+        xs.append(x.download())
+    assert _relerr(xs[0], xs[1]) < 1e-10
