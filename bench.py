@@ -9,11 +9,13 @@ Euler equations on that box (freestream M 0.3 with a seeded Gaussian density
 bump, farfield boundaries), its Jacobian assembled on the device by the DG
 restatement, the pseudo-transient term at cfl 10 added, b = -R(q0).
 
-Prints one JSON line (rank 0).  `value` times the solves with A and b resident
+Prints one JSON line (rank 0) on stdout, and on stderr a line `details {...}` with
+the kernels' times and the legs' results.  `value` times the solves with A and b resident
 in HBM; `e2e` times the same solves through the C ABI from pinned host
 buffers, host->device upload of A and b and download of x included in every
 step, with two pipelines taking alternate steps so that one step's upload
-overlaps the other's solve (`e2e.sequential`: one pipeline, no overlap).
+overlaps the other's solve (`e2e.sequential` of the details: one pipeline, no
+overlap).
 `--impl reference` times the CPU FP64 oracle (the restatement of the
 reference solver; the Fortran original cannot be built here) solving the same
 24^3 system, one whole solve per step, on every host thread.  The GPU arm's
@@ -1339,24 +1341,34 @@ def run_gpu(args):
     achieved = dbytes / (dms / 1e3) / 1e9
     traffic = measured_traffic(dom_key, pat) if args.schedule == "stream" else None
     lat_sorted = sorted(lat_ms)
+    # one short line on stdout (readers keep the end of a run's output); the legs
+    # and the kernels' times on stderr
+    dig = lambda x: float(f"{x:.6g}") if isinstance(x, float) else x
+    short = workload_config()
+    short.update({"precision": "fp64", "ilu_schedule": args.schedule, "fgmres_iterations": sorted(set(niters)),
+                  "true_rel_residual": dig(resid),
+                  "rel_err_vs_oracle": dig(oracle_check["rel_err_vs_oracle"]) if oracle_check else None})
     line = {
         "metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": elapsed_ms / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-        "config": workload_config({"precision": "fp64", "ilu_schedule": args.schedule, "fgmres_iterations": niters,
-                                   "bump_centre": [float(c) for c in centre], "device_assembly_s": assembly_s,
-                                   "true_rel_residual": resid, "stream_shapes": tuned, "autotune_s": tune_s,
-                                   "rel_err_vs_oracle": oracle_check["rel_err_vs_oracle"] if oracle_check else None}),
-        "oracle_check": oracle_check,
-        "latency_ms": {"p50": float(np.percentile(lat_sorted, 50)), "p99": float(np.percentile(lat_sorted, 99))},
+        "config": short,
+        "latency_ms": {"p50": dig(float(np.percentile(lat_sorted, 50))), "p99": dig(float(np.percentile(lat_sorted, 99)))},
         "clocks": clk,
         "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": int(nval * 8 + n * 8),
-                "d2h_bytes_per_step": int(n * 8), "steps": nb_e2e, "pipelines": 2,
-                "sequential": {"value": e2e_seq_value, "steps": nb_seq}, "lanes_x_rel_diff": e2e_x_agree},
+                "d2h_bytes_per_step": int(n * 8)},
         "gpu_launches": launches,
-        "roofline": {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                     "frac": achieved / hbm, "traffic": traffic, "peak_kind": peak_kind,
-                     "algorithmic_bytes_per_launch": dbytes},
+        "roofline": {"kernel": dom, "bound": "hbm", "achieved": dig(achieved), "peak": hbm, "unit": "GB/s",
+                     "frac": dig(achieved / hbm), "peak_kind": peak_kind},
+        "mixed_speedup_vs_fp64": {k: dig(v["speedup_vs_fp64"]) for k, v in mixed.items()},
+    }
+    details = {
+        "config": workload_config({"bump_centre": [float(c) for c in centre], "device_assembly_s": assembly_s,
+                                   "stream_shapes": tuned, "autotune_s": tune_s}),
+        "oracle_check": oracle_check,
+        "e2e": {"steps": nb_e2e, "pipelines": 2, "sequential": {"value": e2e_seq_value, "steps": nb_seq},
+                "lanes_x_rel_diff": e2e_x_agree},
+        "roofline": {"traffic": traffic, "algorithmic_bytes_per_launch": dbytes},
         "kernels": kernels,
         "mixed": mixed,
         "batch": batch,
@@ -1369,6 +1381,7 @@ def run_gpu(args):
         "cfg4": cfg4,
         "cpu_baseline": cpu,
     }
+    print("details " + json.dumps(details), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
     return 0
 
