@@ -207,9 +207,12 @@ __device__ __forceinline__ void sum_partials(const double* partial, int ncta, in
 // own, one CTA taking the sums one after another, was 11 us a pass at 30
 // vectors.  An Arnoldi step of a 6 x 7 x 5 harmonic-balance box of order 1
 // takes 12 us less with the three reductions inside the passes and the scaling
-// not waiting for the host.)
+// not waiting for the host.)  Bound by the reads: 1.87 M entries, 16 vectors 72 us, 30
+// 118 us, of them 71 at the copy rate.  The launch bounds matter: for any block
+// size the compiler keeps fewer loads in flight (107 and 188 us; with sums in
+// launches of their own 93 and 149).
 template <typename T>
-__global__ void k_mdot(int64_t n, const T* __restrict__ x, const T* __restrict__ y, int64_t ystride, int nq,
+__global__ void __launch_bounds__(256, 4) k_mdot(int64_t n, const T* __restrict__ x, const T* __restrict__ y, int64_t ystride, int nq,
                        double* __restrict__ partial, double* out, const double* __restrict__ rows, int nrow,
                        double* row_out, unsigned* counter) {
     // eight vectors per pass over x: x[i] is read once for the eight, and the
