@@ -2232,7 +2232,7 @@ static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV*
 // (comparison runs).
 namespace {
 std::mutex g_shape_mu;
-StreamShape g_shape[kShapeKinds][kShapeClasses][3];
+StreamShape g_shape[kShapeKinds][kShapeClasses][3], g_default[kShapeKinds][kShapeClasses][3];
 bool g_shape_init = false;
 int width_slot(int esz) { return esz >= 8 ? 0 : esz == 4 ? 1 : 2; }
 void init_shapes() {
@@ -2251,6 +2251,7 @@ void init_shapes() {
             g_shape[kShapeBackward][c][w] = given ? sweep : def;
             g_shape[kShapeBackwardMv][c][w] = def;
             g_shape[kShapeMatvec][c][w] = StreamShape{8, 2, 24 * 1024, true};
+            for (int k = 0; k < kShapeKinds; ++k) g_default[k][c][w] = g_shape[k][c][w];
         }
     g_shape_init = true;
 }
@@ -2268,7 +2269,12 @@ StreamShape chidg::stream_shape_for(int kind, int max_b, int esz, bool diagonal)
 void chidg::set_stream_shape(int kind, int max_b, int esz, const StreamShape& sh) {
     std::lock_guard<std::mutex> lk(g_shape_mu);
     if (!g_shape_init) init_shapes();
-    g_shape[kind][shape_class(max_b)][width_slot(esz)] = sh;
+    const int c = shape_class(max_b), w = width_slot(esz);
+    StreamShape& at = g_shape[kind][c][w];
+    at = sh;
+    // the default set again (read, other shapes tried, put back) is the default
+    const StreamShape& d = g_default[kind][c][w];
+    at.standard = d.standard && sh.cw == d.cw && sh.nstage == d.nstage && sh.stage_bytes == d.stage_bytes;
 }
 int chidg::resident_ctas(const void* func, int threads, size_t smem) {
     static std::mutex mu;

@@ -9,7 +9,7 @@ to take all slices of one."""
 import numpy as np
 import pytest
 
-from chidg_b200 import _lib, api, mesh
+from chidg_b200 import _lib, api, mesh, tuning
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -223,7 +223,10 @@ def test_grouped_slices_give_the_sums_of_single_ones(b):
 def test_rows_of_very_many_blocks():
     """One element with 240 time levels of 64 equations: the matvec rows of the
     backward sweep stage 15 360 columns, beside which four stages of the default
-    ring do not fit.  Against the sweeps without matvec rows."""
+    ring do not fit.  Against the sweeps without matvec rows.  (A default that was
+    read and set again is still a default.)"""
+    for kind in range(4):
+        tuning.set_shape(kind, 64, 8, tuning.get_shape(kind, 64, 8))
     pat = mesh.box_pattern(1, 1, 1, 8, 8, ntime=240)
     A = api.ChidgMatrix(pat)
     A.upload(mesh.synth_values(pat, seed=91))
