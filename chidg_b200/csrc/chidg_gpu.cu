@@ -1119,6 +1119,7 @@ static int build_hb(const chidg_gpu_matrix* A, IluProgram& P, std::string& err) 
 // blocks, RASILU0/type_RASILU0_recv_dom_comm.f90:59-305 classifies them).
 static int build_rasilu0(const chidg_gpu_matrix* A, IluProgram& P, std::string& err) {
     P = IluProgram();
+    P.subdomains = true;
     if (A->ntime != 1) { err = "rasilu0: single time level only"; return CHIDG_GPU_EINVAL; }
     int nsub = 0;
     for (int e = 0; e < A->nelem; ++e) nsub = std::max(nsub, A->proc[e] + 1);

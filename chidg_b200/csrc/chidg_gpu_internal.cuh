@@ -77,7 +77,10 @@ struct IluProgram {
     int max_row_task_cols = 0;                 // widest segment a one-task row stages
     std::vector<uint8_t> whole_f, whole_b;     // rows that are one task
     bool diagonal = false;                     // no couplings at all (Jacobi, precon_HB)
-    int slices(int b) const { return diagonal ? sweep_slices_diagonal(b) : sweep_slices(b); }
+    bool subdomains = false;                   // RASILU0
+    int slices(int b) const {
+        return diagonal ? sweep_slices_diagonal(b) : subdomains ? sweep_slices_ras(b) : sweep_slices(b);
+    }
     bool no_lower = false;                     // no row has lower entries: the streamed forward sweep is left out
     std::vector<int64_t> base_f, base_u, base_d;
     Buffer d_sf_task, d_sb_task;

@@ -78,7 +78,19 @@ enum { SW_ENTRY = 0, SW_DIAG = 1, SW_ROW = 2, SW_MATVEC = 3 };   // slice of an 
 
 constexpr int SW_ROW_B = 64;      // rows of at most this size are one task (SW_ROW) ...
 constexpr int SW_ROW_COLS = 384;  // ... if their entries' columns fit the staged segment
+// Slices of a block of b rows.  More shorten a hop, but every child of a row adds
+// up its partial sums again.  Forward and backward sweep with matvec rows, us: 320
+// rows, 8^3, eight 267 / 649, four 289 / 679, three 333 / 738; 9 x 9 x 20, eight 700
+// / 1745, four 653 / 1668.  From 161 to 300 rows small boxes and thin ones want
+// eight (200 rows, 4^3: eight 59 / 135, five 62 / 150; 162 rows, 60 elements in a
+// row: an application 598, with four 697), large boxes fewer (162 rows, 9 x 9 x 20:
+// eight 389 / 742, four 291 / 607, whole blocks 380 / 787).
 inline int sweep_slices(int b) { return b <= SW_ROW_B ? 1 : b <= 160 ? 3 : 8; }
+// RASILU0: many subdomains advance side by side, so its levels are long and its chains
+// short; slices of some 80 columns above 160 rows.  Apply, ms, whole blocks / these /
+// eight: 12^3 elements in 64 subdomains, 162 rows 0.79 / 0.78 / 0.97, 243 rows 1.57 /
+// 1.59 / 1.76, 320 rows 2.68 / 2.72 / 2.88; 8^3 in eight, 320 rows 1.23 / 0.74 / 0.79.
+inline int sweep_slices_ras(int b) { return b <= 160 ? sweep_slices(b) : std::min(8, b / 80); }
 // Programmes without couplings (Jacobi, precon_HB) have no chain, but the matvec
 // rows' wait.  Above 160 rows each of their slices is its own task however many
 // there are, which fills the last turn of the CTAs better than whole blocks (1 slice)

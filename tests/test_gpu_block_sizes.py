@@ -192,10 +192,10 @@ def test_product_of_mixed_sizes_with_more_rows_than_ctas():
     assert _relerr(api.chidg_mv(Ag, api.ChidgVector(Ag, x)).download(), Ao.mv(x)) < 1e-13
 
 
-@pytest.mark.parametrize("b", [65, 161])
+@pytest.mark.parametrize("b", [65, 161, 320])
 def test_grouped_slices_give_the_sums_of_single_ones(b):
-    """300 systems side by side: levels of 300 blocks, whose tasks take all three
-    (65 rows) or eight (161) slices of a block.  Bitwise the application of a
+    """300 systems side by side: levels of 300 blocks, whose tasks take all slices of
+    a block (three at 65 rows, eight above 160).  Bitwise the application of a
     system alone, whose tasks take a slice each; one of them against the oracle."""
     one = mesh.box_pattern(2, 1, 1, 1, b)
     union, sys_elem = mesh.concat_patterns([one] * 300)
@@ -238,3 +238,19 @@ def test_rows_of_very_many_blocks():
         solver.solve(A, x, b, api.create_preconditioner("ilu0", schedule=schedule))
         xs.append(x.download())
     assert _relerr(xs[0], xs[1]) < 1e-10
+
+
+@pytest.mark.parametrize("nvars,nterms", [(5, 8), (7, 23), (5, 48), (5, 64)], ids=["b40", "b161", "b240", "b320"])
+def test_subdomain_sweeps_by_block_size(nvars, nterms):
+    """RASILU0 over eight subdomains (one task a row; two, three and four slices)
+    against the oracle.  Tolerance as in test_gpu_edge.py."""
+    pat = mesh.box_pattern(4, 2, 2, nvars, nterms, subdomains=(2, 2, 2))
+    vals = mesh.synth_values(pat, seed=95)
+    Ao, Ag = O.OracleMatrix(pat), api.ChidgMatrix(pat)
+    Ao.set_values(vals)
+    Ag.upload(vals)
+    Mo, Mg = O.OraclePrecon(Ao, "rasilu0"), api.create_preconditioner("rasilu0")
+    Mo.update()
+    Mg.update(Ag)
+    v = mesh.synth_vector(pat.vector_size(), seed=96)
+    assert _relerr(Mg.apply(Ag, api.ChidgVector(Ag, v)).download(), Mo.apply(v)) < 1e-11
