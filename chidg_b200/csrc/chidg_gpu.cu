@@ -1838,13 +1838,16 @@ static int launch_inverse(chidg_gpu_precon* M, int row_begin, int count, int bma
 }
 
 // precon%update for the mixed-precision inner solves (MIXED_FP32, MIXED_BF16):
-// the L and S products in FP32 (SIMT, from the FP32 copy of A), the diagonal
-// inverses in FP64 (the products' D blocks are written in FP64, inverted by the
-// tensor-core kernel and copied to FP32 per wavefront).  Only the FP32 (and
+// the L and S products in FP32 (from the FP32 copy of A), the diagonal
+// inverses in FP64 (the products' D blocks are written in FP64, inverted as in the
+// FP64 factorisation and copied to FP32 per wavefront).  Only the FP32 (and
 // BF16) factors are produced; LD's FP64 L blocks are not.
-// The products run on the tcgen05 tensor cores (k_task_gemm_umma);
-// CHIDG_FACTOR32_MMA=sync selects the mma.sync TF32 kernel and
-// CHIDG_FACTOR32_SIMT=1 the FP32 SIMT products (comparison runs)
+// The products of blocks up to 136 rows run on the tcgen05 tensor cores
+// (k_task_gemm_umma), larger ones on the SIMT tiled kernel, which the FP64
+// products' tensor-core tiles have overtaken: batched solves of orders 1 to 3 with
+// FP32 inner solves run at 0.90 of the FP64 ones.  CHIDG_FACTOR32_MMA=sync selects
+// the mma.sync TF32 kernel and CHIDG_FACTOR32_SIMT=1 the FP32 SIMT products
+// (comparison runs)
 static int factor32_kernel_env() {       // 0 tcgen05, 1 mma.sync, 2 SIMT
     static const int v = [] {
         const char* s = std::getenv("CHIDG_FACTOR32_SIMT");
@@ -2223,7 +2226,10 @@ static int task_sweeps(chidg_gpu_precon* M, const TL* LD, const TU* U, const TV*
 // same whatever the largest block beside it.  Forward sweep and backward sweep
 // with matvec rows within FP64 solves, us, 24 / 26 KB: 24^3 of order 2 1137 / 1207
 // and 3229 / 2957, 12^3 250 / 240 and 555 / 496, 9 x 8 x 10 of order 3 346 / 362
-// and 882 / 851; 20 KB 1160, 249, 357 and 2941, 527, 950.
+// and 882 / 851; 20 KB 1160, 249, 357 and 2941, 527, 950.  25 KB forward (two chunks
+// of 23 columns and four CTAs an SM) is faster at 135 rows, 1034 against 1124 us at
+// 24^3 and 127 against 141 at 8^3, but not at 320 rows (9 x 8 x 10: 375 against
+// 346); the autotuner finds it.
 // Programmes without couplings (Jacobi, precon_HB) have no chain, only as many
 // copies in flight as CTAs fit: their backward sweep takes two stages of 24 KB, four
 // CTAs an SM, and with the matvec rows of blocks up to 64 rows 20 KB (24^3 elements

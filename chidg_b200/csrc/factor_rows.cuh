@@ -16,7 +16,8 @@
 // x 8 1.38, 1.07; 18^3 3.24, 2.35; 24^3 4.80, 3.53; 8 rows 18^3 1.61, 0.70; 54
 // rows 14^3 3.02, 2.62; 64 rows 14^3 3.25, 2.97, 24^3 7.36, 5.99.  Larger blocks
 // keep the three launches: their products are several CTA tiles and their
-// inverse wants more warps than the tile has.
+// inverse wants more warps than the tile has.  With profiling on the launch counts
+// as factorisation only: its products and inverses are not launches of their own.
 #pragma once
 
 #include "factor_gemm.cuh"

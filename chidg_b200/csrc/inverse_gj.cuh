@@ -21,7 +21,7 @@
 //             records its row p_k.
 //   update    every other column c changes by the panel's eight steps as
 //             a_c <- a_c with rows {p_k} zeroed + P X_c, P the eliminated
-//             panel and X_c the old values of a_c in rows p_k: m16n8k8 FP64
+//             panel and X_c the old values of a_c in rows p_k: m8n8k4 FP64
 //             tensor-core products, a warp a tile of eight columns.
 //
 // Look-ahead: the panel warps apply panel J to tile J + 1 themselves (each

@@ -167,9 +167,10 @@ def test_stream_sweeps_mixed_precision(precision, P):
 
 
 @pytest.mark.parametrize("nvars,P", [(3, 2), (4, 2), (1, 4), (2, 3), (5, 2)])
-def test_factor_tensor_core_inverse_sizes(nvars, P):
-    """Diagonal inverses of 81..136-row blocks (blocked Gauss-Jordan on the FP64
-    tensor cores, partial tiles included) against the oracle's DGETRF/DGETRI."""
+def test_factor_inverse_sizes_one_cta(nvars, P):
+    """Diagonal inverses of 81..136-row blocks (panels of eight columns and
+    tensor-core updates by one CTA, partial tiles included) against the oracle's
+    DGETRF/DGETRI."""
     pat, vals, Ao, Ag = setup((3, 2, 2), P, seed=30, nvars=nvars)
     Mo = O.OraclePrecon(Ao, "ilu0")
     Mo.update()
@@ -187,10 +188,10 @@ def test_factor_tensor_core_inverse_sizes(nvars, P):
 
 
 @pytest.mark.parametrize("nvars", [3, 4, 5])
-def test_factor_row_inverse_sizes(nvars):
-    """Diagonal inverses of 192..320-row blocks (P3; Gauss-Jordan with a row
-    of the block per thread and panels in registers) and the L blocks built
-    from them, against the oracle's DGETRF/DGETRI and ILU0."""
+def test_factor_inverse_sizes_clusters(nvars):
+    """Diagonal inverses of 192..320-row blocks (P3; the same panels, by clusters
+    of two to five CTAs) and the L blocks built from them, against the oracle's
+    DGETRF/DGETRI and ILU0."""
     pat, vals, Ao, Ag = setup((2, 2, 1), 3, seed=36, nvars=nvars)
     Mo = O.OraclePrecon(Ao, "ilu0")
     Mo.update()
@@ -211,7 +212,7 @@ def test_factor_row_inverse_sizes(nvars):
 def test_inverse_with_row_permuted_blocks(P):
     """Diagonal blocks whose rows are shuffled, so that partial pivoting takes
     off-diagonal pivots and the inverse kernels undo a long permutation
-    (135 rows: tensor-core kernel; 320 rows: row-per-thread kernel), against
+    (135 rows: one CTA; 320 rows: a cluster of five), against
     the oracle's DGETRF/DGETRI (block Jacobi: the inverses alone)."""
     pat, vals, Ao, Ag = setup((2, 2, 1), P, seed=38)
     voff, _ = pat.value_offsets()
@@ -237,7 +238,7 @@ def test_inverse_with_row_permuted_blocks(P):
     assert worst < 1e-10
 
 
-def test_singular_block_reports_element_row_inverse():
+def test_singular_block_reports_element_cluster_inverse():
     pat, vals, Ao, Ag = setup((2, 2, 1), 3, seed=37)
     voff, _ = pat.value_offsets()
     nr, nc = pat.block_dims()
@@ -252,7 +253,7 @@ def test_singular_block_reports_element_row_inverse():
     assert ei.value.code == _lib.ESINGULAR and ei.value.element == 2
 
 
-def test_singular_block_reports_element_tensor_core_inverse():
+def test_singular_block_reports_element_one_cta_inverse():
     pat, vals, Ao, Ag = setup((3, 2, 2), 2, seed=31)
     voff, _ = pat.value_offsets()
     nr, nc = pat.block_dims()
